@@ -118,9 +118,14 @@ __device__ __forceinline__ uint64_t streamBits(const uint64_t* __restrict__ pack
     return o ? (hi << o) | (__ldg(packed + w + 1) >> (64 - o)) : hi;
 }
 
-// The code of character q.
+// The code of character q: one word of the stream, two when the character straddles them.
 __device__ __forceinline__ uint32_t charCode(const TextSet& texts, uint64_t q) {
-    return static_cast<uint32_t>(streamBits(texts.packed, q * texts.bits) >> (64 - texts.bits));
+    const uint64_t bit = q * texts.bits;
+    const uint32_t end = static_cast<uint32_t>(bit & 63) + texts.bits;
+    const uint64_t* word = texts.packed + (bit >> 6);
+    const uint64_t hi = __ldg(word);
+    const uint64_t code = end <= 64 ? hi >> (64 - end) : (hi << (end - 64)) | (__ldg(word + 1) >> (128 - end));
+    return static_cast<uint32_t>(code) & ((1u << texts.bits) - 1);
 }
 
 // The byte of character q.

@@ -2,15 +2,13 @@
 //
 // The difference cover modulo 32, D = {0, 1, 3, 8, 12, 19, 25} (the cover of the reference's GPU
 // path, src/common/differencecover.h:29-31 and src/cuda/devicecommon.cuh:31-36), with its lookup
-// tables generated at compile time from D and placed in __constant__ memory by static
-// initialisation, so every device that loads the module has them without an upload.
+// tables generated at compile time from D (host); device code works on D's bit mask.
 //
 // Text layout in HBM: the text bytes, 8-byte aligned, followed by kTextPad zero bytes, so that a
 // 16-byte window at any position <= n + 31 stays inside the buffer and reads zeros past the end.
 #pragma once
 
 #include <atomic>
-#include <cstddef>
 #include <cstdint>
 #include <utility>
 #include <cuda_runtime.h>
@@ -23,15 +21,11 @@ constexpr int kClasses = 7;   // distance to the next sample position: 0 (the sa
 constexpr uint32_t kTextPad = 128;
 constexpr uint32_t kRankPad = 16;  // zero rank entries past the sample: a 7-rank window at any p <= n stays inside
 
-// The square tables come first and 16-byte aligned: kernels copy them to shared memory as words.
-struct alignas(16) Cover {
-    alignas(16) uint8_t tie[kV][kV];   // smallest k with a + k and b + k both sampled
-    alignas(16) uint8_t slot[kV][kV];  // [a][k]: index of sample a + k among the samples in [a, a + 32)
+struct Cover {
     uint8_t below[kV];                 // cover residues below r
     uint8_t classOf[kV];               // distance from residue r to the next cover residue
     uint8_t residue[kK];
 };
-static_assert(offsetof(Cover, tie) % 16 == 0 && offsetof(Cover, slot) % 16 == 0, "word copies of the tables");
 
 constexpr bool coverHas(int r) {
     constexpr int d[kK] = {0, 1, 3, 8, 12, 19, 25};
@@ -54,19 +48,6 @@ constexpr Cover makeCover() {
         int d = 0;
         while (!coverHas(r + d)) d++;
         c.classOf[r] = static_cast<uint8_t>(d);
-    }
-    for (int a = 0; a < kV; a++) {
-        for (int b = 0; b < kV; b++) {
-            int t = 0;
-            while (!coverHas(a + t) || !coverHas(b + t)) t++;
-            c.tie[a][b] = static_cast<uint8_t>(t);
-        }
-        for (int t = 0; t < kV; t++) {
-            // samples in [a, a + t) = pack(a + t) - pack(a), with pack over absolute positions
-            int count = 0;
-            for (int q = a; q < a + t; q++) count += coverHas(q) ? 1 : 0;
-            c.slot[a][t] = static_cast<uint8_t>(count);
-        }
     }
     return c;
 }
@@ -97,8 +78,6 @@ __device__ __forceinline__ uint32_t sampleSlot(uint32_t rotA, uint32_t k) {
     return static_cast<uint32_t>(__popc(rotA & ((1u << k) - 1)));
 }
 static_assert(kCoverTables.classOf[2] == 1 && kCoverTables.classOf[26] == 6, "cover tables");
-
-__constant__ Cover cCover = makeCover();
 
 // Number of sample positions below p: a sample position's index in the compact rank array.
 inline uint64_t packHost(uint64_t p) {

@@ -1,7 +1,7 @@
 // merge.cuh - one multiway merge of the 7 sorted class lists into the suffix array and the BWT
 // (the reference's step 4, src/cuda/merge.cuh; comparison as lessGlobal, merge.cuh:53-71).
 //
-// Two suffixes i, j compare in O(1): k = tie[i%32][j%32] < 32 has i + k and j + k both sampled, so
+// Two suffixes i, j compare in O(1): the cover's tie offset k < 32 has i + k and j + k both sampled, so
 // compare T[i, i+k) with T[j, j+k) and then the sample ranks at i + k and j + k; a suffix that ends
 // first is the smaller.
 //
@@ -58,9 +58,29 @@ __host__ __device__ constexpr uint32_t mergeR(int words) {
 __host__ __device__ constexpr int mergeThreads(int words) {
     return words == 1 ? SADCS_MERGE_THREADS_W1 : SADCS_MERGE_THREADS;
 }
+
+// Tile shape of the kernel for texts with few long repeats (merge_wide.cuh): C outputs per thread and
+// tree level, and as many records as the threads then take with one ragged thread per merge of a
+// level. C is odd, so that the threads' stores of consecutive 8-byte entries touch every bank pair.
+// Final level at C = 7 with 256 threads, 4 tiles per SM: 69.0 ms for the 4096-text batch, 2.39 for 100 MB
+// of protein-like text; C = 5: 73.8 and 2.51; 384 threads, C = 5: 71.2 and 2.51; 192 threads, C = 5: 80.8
+// and 2.77 (tuning).
+#ifndef SADCS_WIDE_THREADS
+#define SADCS_WIDE_THREADS 256
+#endif
+#ifndef SADCS_WIDE_ITEMS
+#define SADCS_WIDE_ITEMS 7
+#endif
+#ifndef SADCS_WIDE_TILES
+#define SADCS_WIDE_TILES 4
+#endif
+constexpr uint32_t kWideR = ((SADCS_WIDE_THREADS - 3) * SADCS_WIDE_ITEMS - 6 * (kMergeG - 1) - 1) / kMergeG;
+static_assert(mergeCap(kWideR) + 2 * (SADCS_WIDE_ITEMS - 1) <= SADCS_WIDE_THREADS * SADCS_WIDE_ITEMS,
+              "threads for every output of a level's (at most 3) merges");
 // The smallest R of any shape: the most rows a plan can have (memory plans bound with it).
-constexpr uint32_t kMergeRMin = SADCS_MERGE_R < SADCS_MERGE_R_W1 ? SADCS_MERGE_R : SADCS_MERGE_R_W1;
-static_assert(mergeCap(SADCS_MERGE_R) <= 65535 && mergeCap(SADCS_MERGE_R_W1) <= 65535, "u16 record indices");
+constexpr uint32_t kMergeRMin = std::min({mergeR(1), mergeR(2), kWideR});
+static_assert(mergeCap(mergeR(2)) <= 65535 && mergeCap(mergeR(1)) <= 65535 && mergeCap(kWideR) <= 65535,
+              "u16 record indices");
 constexpr uint32_t kNoList = 0xFFFFFFFFu;
 constexpr int kMaxLevels = 10;
 
@@ -70,24 +90,12 @@ struct __align__(16) MergeRow {
 };
 static_assert(sizeof(MergeRow) == 32, "a row is 8 words");
 
-// A suffix for single comparisons in registers (the searches of mergeSuffixZeroRows): w0, w1 = 128
-// bits of the code stream from pos; end: the end of pos's text (texts are ordered by it); text: its
-// index. Comparisons reaching past w1 read the code stream.
-struct MergeRecord {
-    uint64_t w0, w1;
-    uint32_t rank[kK];
-    uint32_t pos;
-    uint32_t end;
-    uint32_t text;
-};
-
 struct MergeLevel {
     const uint32_t* lists;
     uint32_t start[kClasses + 1];
 };
 
 struct MergeArgs {
-    const uint8_t* text;
     const uint32_t* ranks;
     TextSet texts;
     MergeLevel level;
@@ -102,6 +110,8 @@ struct MergeArgs {
     uint32_t* error;         // set nonzero if a window set exceeds the capacity (never, by construction)
     const uint64_t* carried;  // level 0, optional: every list slot's carried word (one text, 1-word records)
     uint32_t tileOffset;      // tiles of this launch start here (a level launched in pieces)
+    uint32_t span;            // positions are below it
+    uint32_t wide;            // nonzero: the kernel for texts with few long repeats (merge_wide.cuh)
 };
 
 // The top `bits` bits set (bits <= 64).
@@ -109,76 +119,46 @@ __device__ __forceinline__ uint64_t topMask(uint32_t bits) {
     return bits >= 64 ? ~uint64_t(0) : (bits == 0 ? uint64_t(0) : ~uint64_t(0) << (64 - bits));
 }
 
-__device__ __forceinline__ void loadRecord(const uint8_t* __restrict__ text, const uint32_t* __restrict__ ranks,
-                                           const TextSet& texts, uint32_t p, MergeRecord& r) {
-    const uint64_t bit = static_cast<uint64_t>(p) * texts.bits;
-    r.w0 = streamBits(texts.packed, bit);
-    r.w1 = streamBits(texts.packed, bit + 64);
-    const uint32_t base = pack(p);
-#pragma unroll
-    for (int s = 0; s < kK; s++) r.rank[s] = __ldg(ranks + base + s);
-    r.pos = p;
-    r.text = texts.textOf(p);
-    r.end = texts.endOfText(r.text);
+// Suffixes i and j of one text ending at n, whose first `held` stream bits are known to agree: the
+// rest of their first `common` characters, -1 or 1 for the order they give, 0 if they agree too.
+__device__ __forceinline__ int streamOrder(const TextSet& texts, uint32_t i, uint32_t j, uint32_t held,
+                                           uint32_t common) {
+    const uint32_t stop = common * texts.bits;
+    for (uint32_t o = held; o < stop; o += 64) {
+        const uint64_t mask = topMask(stop - o);
+        const uint64_t x = streamBits(texts.packed, static_cast<uint64_t>(i) * texts.bits + o) & mask;
+        const uint64_t y = streamBits(texts.packed, static_cast<uint64_t>(j) * texts.bits + o) & mask;
+        if (x != y) return x < y ? -1 : 1;
+    }
+    return 0;
 }
 
-// Cover tables the comparison reads, in shared memory: the threads of a warp index them at
-// different places, which constant memory would serialise.
-struct MergeTables {
-    uint8_t tie[kV][kV];
-    uint8_t slot[kV][kV];
-};
-
-__device__ __forceinline__ bool lessRecord(const MergeRecord& a, const MergeRecord& b, const TextSet& texts,
-                                           const MergeTables& tb) {
-    if (a.end != b.end) return a.end < b.end;  // different texts: text order
-    const uint32_t n = a.end;
-    const uint32_t i = a.pos, j = b.pos;
-    const uint32_t k = tb.tie[i % kV][j % kV];
-    const uint32_t common = min(k, min(n - i, n - j));
-    const uint32_t bits = common * texts.bits;
-    uint64_t x = a.w0, y = b.w0;
-    if (bits < 64) {
-        const uint64_t mk = topMask(bits);
-        x &= mk;
-        y &= mk;
-    }
-    if (x != y) return x < y;
-    if (bits > 64) {
-        x = a.w1;
-        y = b.w1;
-        if (bits < 128) {
-            const uint64_t mk = topMask(bits - 64);
-            x &= mk;
-            y &= mk;
-        }
-        if (x != y) return x < y;
-        for (uint32_t o = 128; o < bits; o += 64) {
-            x = streamBits(texts.packed, static_cast<uint64_t>(i) * texts.bits + o);
-            y = streamBits(texts.packed, static_cast<uint64_t>(j) * texts.bits + o);
-            if (bits - o < 64) {
-                const uint64_t mk = topMask(bits - o);
-                x &= mk;
-                y &= mk;
-            }
-            if (x != y) return x < y;
-        }
-    }
-    if (common < k || i + k == n || j + k == n) return i > j;  // one is a prefix of the other
-    return a.rank[tb.slot[i % kV][k]] < b.rank[tb.slot[j % kV][k]];
+// Suffix i < suffix j of one text ending at n, whose first `held` stream bits are known to agree: the
+// rest of their first k characters (k the cover's tie offset; fewer where one of them ends), then the
+// lengths when one ends within k, else the sample ranks at i + k and j + k.
+__device__ __forceinline__ bool suffixLess(const uint32_t* __restrict__ ranks, const TextSet& texts, uint32_t n,
+                                           uint32_t i, uint32_t j, uint32_t held) {
+    const uint32_t k = tieOffset(coverRotation(i), coverRotation(j));
+    const uint32_t shorter = min(n - i, n - j);
+    if (const int order = streamOrder(texts, i, j, held, min(k, shorter))) return order < 0;
+    if (k >= shorter) return i > j;  // one is a prefix of the other
+    return __ldg(ranks + pack(i + k)) < __ldg(ranks + pack(j + k));
 }
 
 struct MergeTileInfo {
     uint32_t seg[kClasses + 1];
     uint32_t win[kClasses];
+    uint32_t slot[kClasses];  // record e of list b is element slot[b] + e of the level's lists (mod 2^32)
     uint32_t base, loIdx, hiIdx, size;
     int bad;
 };
 
 
-__device__ __forceinline__ int listOfElement(const uint32_t* seg, uint32_t e) {
-    int l = 0;
-    while (e >= seg[l + 1]) l++;
+// The list of record e (below seg[kClasses]).
+__device__ __forceinline__ uint32_t listOfElement(const uint32_t* seg, uint32_t e) {
+    uint32_t l = 0;
+#pragma unroll
+    for (int b = 1; b < kClasses; b++) l += e >= seg[b] ? 1u : 0u;
     return l;
 }
 
@@ -233,6 +213,7 @@ __device__ __forceinline__ void planTileWindows(const MergeArgs& a, uint32_t cap
     if (b < kClasses) {
         t.win[b] = w;
         t.seg[b + 1] = seg;
+        t.slot[b] = st[b] + w - (seg - (e - w));
     }
     if (b == 0) {
         t.seg[0] = 0;
@@ -263,41 +244,33 @@ __global__ void mergeWriteSentinel(MergeRow* row, MergeLevel level) {
     }
 }
 
-// rowZero[j] += the elements of list threadIdx.x in text j smaller than text j's first suffix: its
-// output row within the text. One block per text. rowBase: the class tables' first slot of every
-// (class, text); classEnd: plan.start[1..7].
-__global__ void mergeSuffixZeroRows(MergeArgs a, const uint32_t* __restrict__ rowBase, MergeLevel classes,
-                                    uint32_t* rowZero) {
-    __shared__ MergeTables tb;
-    for (int i = threadIdx.x; i < kV * kV; i += blockDim.x) {
-        (&tb.tie[0][0])[i] = (&cCover.tie[0][0])[i];
-        (&tb.slot[0][0])[i] = (&cCover.slot[0][0])[i];
-    }
-    __syncthreads();
-    const int b = threadIdx.x;
+// rowZero[j] += the elements of list b in text j smaller than text j's first suffix: its output row
+// within the text. One block per text, one warp per list: 32 probes of the list a step, so a list
+// of n elements takes log32(n) dependent reads. rowBase: the class tables' first slot of every
+// (class, text); classes: the class lists' offsets.
+__global__ void __launch_bounds__(32 * kClasses) mergeSuffixZeroRows(MergeArgs a, const uint32_t* __restrict__ rowBase,
+                                                                     MergeLevel classes, uint32_t* rowZero) {
+    const uint32_t lane = threadIdx.x & 31, b = threadIdx.x >> 5;
     const uint32_t j = blockIdx.x, J = a.texts.count;
-    if (b >= kClasses) return;
-    MergeRecord zero;
-    loadRecord(a.text, a.ranks, a.texts, a.texts.startOf(j), zero);
+    const uint32_t zero = a.texts.startOf(j), end = a.texts.endOfText(j);
     const uint32_t first = rowBase[static_cast<size_t>(b) * J + j];
     const uint32_t last = j + 1 < J ? rowBase[static_cast<size_t>(b) * J + j + 1] : classes.start[b + 1];
     const uint32_t* list = a.level.lists + first;
     uint32_t lo = 0, hi = last - first;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        MergeRecord r;
-        loadRecord(a.text, a.ranks, a.texts, list[mid], r);
-        if (lessRecord(r, zero, a.texts, tb)) {
-            lo = mid + 1;
-        } else {
-            hi = mid;
-        }
+    while (lo < hi) {  // elements below lo are smaller, elements from hi on are not (warp-uniform)
+        const uint32_t stride = (hi - lo + 31) / 32;
+        const uint64_t at = lo + static_cast<uint64_t>(lane) * stride;
+        const bool less = at < hi && suffixLess(a.ranks, a.texts, end, list[at], zero, 0);
+        const uint32_t smaller = __popc(__ballot_sync(0xffffffffu, less));  // the first probes, by order
+        if (smaller == 0) break;
+        hi = static_cast<uint32_t>(min(static_cast<uint64_t>(hi), lo + static_cast<uint64_t>(smaller) * stride));
+        lo += (smaller - 1) * stride + 1;
     }
-    atomicAdd(rowZero + j, lo);
+    if (lane == 0 && lo) atomicAdd(rowZero + j, lo);
 }
 
 // bwt[outBase[j]] = the last character of text j (the sentinel's row).
-__global__ void mergeBwtHeads(const uint8_t* __restrict__ text, TextSet texts, const uint32_t* __restrict__ outBase,
+__global__ void mergeBwtHeads(TextSet texts, const uint32_t* __restrict__ outBase,
                               uint8_t* bwt, uint8_t* const* bwtTexts) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= texts.count) return;
@@ -320,7 +293,7 @@ struct MergePlan {
     size_t rows = 0;
 };
 
-// r: the tile shape's row spacing (mergeR of the texts' code width).
+// r: the tile shape's row spacing (mergeR of the texts' code width, or kWideR).
 inline MergePlan planMerge(const uint32_t* classStart, uint32_t r) {
     MergePlan p;
     for (int b = 0; b <= kClasses; b++) p.start[0][b] = classStart[b];
@@ -392,9 +365,9 @@ inline cudaError_t copyDown(const OverlappedDownload& d, uint64_t from, uint64_t
 }
 
 // Merges the class lists of the texts into sa and/or bwt (either may be null). splitters and rows
-// are scratch sized by planMerge; counter is one device word (scratch); rowZero and outBase are per
+// are scratch sized by planMerge; counter is one device word (scratch); wide: the kernel for texts with few long repeats; rowZero and outBase are per
 // text (rowZero is filled here when a BWT is asked for); rowBase: the class tables' row bases.
-inline cudaError_t mergeClasses(const uint8_t* text, const uint32_t* ranks, const TextSet& texts, const uint32_t* lists,
+inline cudaError_t mergeClasses(uint32_t span, bool wide, const uint32_t* ranks, const TextSet& texts, const uint32_t* lists,
                                 const MergePlan& plan, const uint32_t* rowBase, const uint32_t* outBase,
                                 uint32_t* rowZero, uint32_t* splitters, MergeRow* rows, uint32_t* sa, uint8_t* bwt,
                                 uint32_t* counter, uint32_t* hostWord, cudaStream_t stream,
@@ -413,7 +386,8 @@ inline cudaError_t mergeClasses(const uint8_t* text, const uint32_t* ranks, cons
     }
     SADCS_TRY(cudaMemsetAsync(counter, 0, sizeof(uint32_t), stream));  // error word
     MergeArgs base{};
-    base.text = text;
+    base.span = span;
+    base.wide = wide;
     base.ranks = ranks;
     base.texts = texts;
     base.outBase = outBase;
@@ -425,8 +399,8 @@ inline cudaError_t mergeClasses(const uint8_t* text, const uint32_t* ranks, cons
         MergeArgs z = base;
         z.level = level[0];
         SADCS_TRY(cudaMemsetAsync(rowZero, 0, sizeof(uint32_t) * texts.count, stream));
-        SADCS_TRY(launch(mergeSuffixZeroRows, texts.count, 32, 0, stream, z, rowBase, level[0], rowZero));
-        SADCS_TRY(launch(mergeBwtHeads, (texts.count + 255) / 256, 256, 0, stream, text, texts, outBase, bwt, bwtTexts));
+        SADCS_TRY(launch(mergeSuffixZeroRows, texts.count, 32 * kClasses, 0, stream, z, rowBase, level[0], rowZero));
+        SADCS_TRY(launch(mergeBwtHeads, (texts.count + 255) / 256, 256, 0, stream, texts, outBase, bwt, bwtTexts));
     }
     for (int L = plan.top; L >= 0; L--) {
         MergeArgs args = base;

@@ -1,4 +1,5 @@
-// merge_final.cuh - the merge levels: every tile of the 7 lists of a level merged in shared memory;
+// merge_final.cuh - the merge levels (texts whose codes take more than one record word and that have few
+// long repeats go to merge_wide.cuh instead: useWideMerge): every tile of the 7 lists of a level merged in shared memory;
 // the last level writes the suffix array and the BWT, an upper level the rows of the level below.
 //
 // A tile's window set (at most kMergeCap records, merge.cuh) is held as arrays of fields, not as
@@ -18,6 +19,7 @@
 #pragma once
 
 #include "merge.cuh"
+#include "merge_wide.cuh"
 
 namespace sadcs {
 
@@ -271,11 +273,11 @@ __device__ __forceinline__ void mergeTileTail(const MergeArgs& a, const FinalTil
                 continue;
             }
             const uint32_t x = order[r];
-            const int l = listOfElement(t.seg, x);
+            const uint32_t l = listOfElement(t.seg, x);
             MergeRow row;
-            row.list = static_cast<uint32_t>(l);
+            row.list = l;
 #pragma unroll
-            for (int b = 0; b < kClasses; b++) {
+            for (uint32_t b = 0; b < kClasses; b++) {
                 if (b == l) {
                     row.c[b] = t.win[l] + (x - t.seg[l]);
                     continue;
@@ -347,7 +349,7 @@ __global__ void __launch_bounds__(mergeThreads(W), mergeTilesPerSm<W>()) mergeTr
                     p[j] = 0;
                     c[j] = 0;
                     if (h + j < kItems && e < size) {
-                        const int l = listOfElement(t.seg, e);
+                        const uint32_t l = listOfElement(t.seg, e);
                         const uint32_t slot = st[l] + t.win[l] + (e - t.seg[l]);
                         p[j] = a.level.lists[slot];
                         c[j] = a.carried[slot];
@@ -386,7 +388,7 @@ __global__ void __launch_bounds__(mergeThreads(W), mergeTilesPerSm<W>()) mergeTr
         const uint32_t e = threadIdx.x + j * kMergeThreads;
         p[j] = 0;
         if (e < size) {
-            const int l = listOfElement(t.seg, e);
+            const uint32_t l = listOfElement(t.seg, e);
             p[j] = a.level.lists[st[l] + t.win[l] + (e - t.seg[l])];
         }
     }
@@ -478,9 +480,26 @@ inline cudaError_t launchTreeWidth(const MergeArgs& args, uint32_t tiles, cudaSt
     }
 }
 
+// Whether a construction merges with merge_wide.cuh's kernel. deep: the samples that still shared
+// their first 20 characters or more with another (RankStats). That kernel compares a few words per
+// record cheaply and puts records that agree in all of them in order afterwards, one tile phase more;
+// this one decides such ties where they are met. Final level with few ties (deep = 0): the
+// 4096-text batch 69.0 ms against 130.8 here, 100 MB of protein-like text 2.39 against 3.03, 8 MiB of
+// uniform bytes 0.213 against 0.303; with many: 256 MiB of natural-language-like text (a third of
+// its samples deep) 17.3 against 14.95, 48 MiB of versions of one document 6.0 against 2.1. The
+// narrow codes' one-word records (a key alone) gain nothing and lose on repeats (2 GiB of genome-like
+// text 58-70 ms against 48.2), so they stay here.
+inline bool useWideMerge(uint32_t bits, uint64_t deep, uint64_t samples) {
+    return finalWords(bits) > 1 && deep <= samples / 32;
+}
+
 // One merge level: kFinal writes the SA and BWT, otherwise the rows of the level below.
 template <bool kFinal>
 inline cudaError_t launchTree(const MergeArgs& args, uint32_t tiles, cudaStream_t stream) {
+    if (args.wide) {
+        return args.texts.count > 1 ? launchWide<true, kFinal>(args, tiles, stream)
+                                    : launchWide<false, kFinal>(args, tiles, stream);
+    }
     return args.texts.count > 1 ? launchTreeWidth<true, kFinal>(args, tiles, stream)
                                 : launchTreeWidth<false, kFinal>(args, tiles, stream);
 }

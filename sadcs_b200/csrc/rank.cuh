@@ -485,9 +485,11 @@ inline uint32_t firstPassChars(const TextSet& texts, uint64_t samples) {
     return texts.keyChars;
 }
 
+constexpr uint64_t kDeepChars = 20;
 struct RankStats {
     int characterPasses = 0;
     int doublingRounds = 0;
+    uint64_t deep = 0;  // samples that shared their first kDeepChars characters or more with another
 };
 
 // Ranks the live sample suffixes of the texts. slots = rank entries (sample positions of the whole
@@ -584,6 +586,7 @@ inline cudaError_t rankSample(const uint8_t* text, const TextSet& texts, uint32_
             stats.characterPasses++;
             depth += passTexts.keyChars;
         }
+        if (depth >= kDeepChars && stats.deep == 0) stats.deep = u;
         first = false;
     }
     return cudaSuccess;

@@ -723,8 +723,9 @@ int construct(sadcs_gpu_context* c, const Batch& b, Io& io, cudaStream_t stream,
     uint32_t* sa = saPieces ? nullptr
                             : (io.outSa ? io.outSa : (io.wantSa ? reinterpret_cast<uint32_t*>(slab + L.sa) : nullptr));
     uint8_t* bwt = bwtPieces ? nullptr : (io.outBwt ? io.outBwt : (io.wantBwt ? slab + L.bwt : nullptr));
-    // The merge's tile shape follows the code width, known now (the memory plan bounds every shape).
-    const MergePlan mergePlan = planMerge(b.classes.start, mergeR(finalWords(texts.bits)));
+    // The merge's kernel and tile shape follow the code width and the ties, known now (the memory plan bounds every shape).
+    const bool wide = useWideMerge(texts.bits, rankStats.deep, b.live);
+    const MergePlan mergePlan = planMerge(b.classes.start, wide ? kWideR : mergeR(finalWords(texts.bits)));
     OverlappedDownload download;
     const bool overlapped = (io.hostSa || io.hostBwt) && c->copyStream;
     if (overlapped) {
@@ -737,7 +738,7 @@ int construct(sadcs_gpu_context* c, const Batch& b, Io& io, cudaStream_t stream,
         download.hostRows = c->hostWords + 64;  // the tables' staging words, free since their upload
         download.outputs = b.outputs;
     }
-    if ((error = mergeClasses(text, ranks, texts, lists, mergePlan, classTables.rowBase, dOutBase, dRowZero,
+    if ((error = mergeClasses(J == 1 ? b.end[0] : b.end[J - 1], wide, ranks, texts, lists, mergePlan, classTables.rowBase, dOutBase, dRowZero,
                               reinterpret_cast<uint32_t*>(slab + L.splitters),
                               reinterpret_cast<MergeRow*>(slab + L.rows), sa, bwt,
                               reinterpret_cast<uint32_t*>(slab + L.mergeCounter), c->hostWords, stream,
