@@ -223,7 +223,7 @@ void sadcs_gpu_server_destroy(sadcs_gpu_server* server);
 
 /* No counterpart: the reference's BWT check (src/common/checker.cpp:196-245) on the device: inverts
  * d_bwt (n bytes, primary) and compares with d_text. *bad_index = -1 if correct, else the first text
- * position that differs (0 if the BWT does not invert at all). Uses about 25n bytes of temporary
+ * position that differs (0 if the BWT does not invert at all). Uses about 7n bytes of temporary
  * device memory. */
 int sadcs_gpu_check_bwt(const uint8_t* d_text, int64_t n, const uint8_t* d_bwt, int64_t primary, int64_t* bad_index,
                         void* stream);
@@ -239,7 +239,7 @@ int sadcs_gpu_check_suffix_array_host(const uint8_t* text, int64_t n, const uint
 /* checkBwt (src/common/checker.h:29, checker.cpp:196-245) with host buffers: text and bwt (n bytes
  * each) and primary, checked on the device by sadcs_gpu_check_bwt. *bad_index = -1 if the BWT
  * inverts to the text, else the first text position where it does not (0 if it does not invert).
- * Uses about 27n bytes of temporary device memory. */
+ * Uses about 9n bytes of temporary device memory. */
 int sadcs_gpu_check_bwt_host(const uint8_t* text, int64_t n, const uint8_t* bwt, int64_t primary, int64_t* bad_index);
 
 /* No counterpart: the inverse BWT (unbwt) on the device: d_text (n bytes) from d_bwt and primary.
