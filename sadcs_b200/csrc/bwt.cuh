@@ -24,7 +24,7 @@ __global__ void bwtGather(const uint8_t* __restrict__ text, const uint32_t* __re
 }
 
 inline cudaError_t bwtFromSa(const uint8_t* text, uint32_t n, const uint32_t* sa, uint8_t* bwt, uint32_t* row0Device,
-                             uint32_t* hostWord, cudaStream_t stream, uint32_t* row0) {
+                             cudaStream_t stream, uint32_t* row0) {
     if (n == 0) {
         *row0 = 0;
         return cudaSuccess;
@@ -32,10 +32,8 @@ inline cudaError_t bwtFromSa(const uint8_t* text, uint32_t n, const uint32_t* sa
     SADCS_TRY(cudaMemsetAsync(row0Device, 0, sizeof(uint32_t), stream));
     SADCS_TRY(launch(bwtFindZero, (n + 255) / 256, 256, 0, stream, sa, n, row0Device));
     SADCS_TRY(launch(bwtGather, (n + 255) / 256, 256, 0, stream, text, sa, n, row0Device, bwt));
-    SADCS_TRY(cudaMemcpyAsync(hostWord, row0Device, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-    SADCS_TRY(cudaStreamSynchronize(stream));
-    *row0 = *hostWord;
-    return cudaSuccess;
+    SADCS_TRY(cudaMemcpyAsync(row0, row0Device, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
+    return cudaStreamSynchronize(stream);
 }
 
 }  // namespace sadcs

@@ -347,7 +347,60 @@ void destroyContext(sadcs_gpu_context* c) {
     delete c;
 }
 
-int queryDevice(sadcs_gpu_device* device) {
+// Temporary device memory of the calls that take no context (checks, LCP array, inverse BWT, gather): a
+// stream-ordered pool per device that keeps up to kWorkspaceKeep bytes between calls, so that a call
+// does not map and unmap its memory each time (at 128 MiB the LCP array took 18-23 ms a call, 11 of
+// them on the device, with the default pool, which gives everything back at every
+// synchronisation). Whatever is kept is given back before free memory is reported (sadcs_gpu_query_device),
+// counted for a server, or found too little for a context. The pool itself is safe across threads and
+// streams.
+constexpr uint64_t kWorkspaceKeep = uint64_t(2) << 30;
+constexpr int kWorkspaceDevices = 64;
+std::mutex gWorkspaceLock;
+cudaMemPool_t gWorkspacePool[kWorkspaceDevices] = {};
+
+cudaError_t workspacePool(cudaMemPool_t* pool, bool create) {
+    *pool = nullptr;
+    int device = 0;
+    cudaError_t error = cudaGetDevice(&device);
+    if (error != cudaSuccess) return error;
+    if (device < 0 || device >= kWorkspaceDevices) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> hold(gWorkspaceLock);
+    if (!gWorkspacePool[device] && create) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t made = nullptr;
+        uint64_t keep = kWorkspaceKeep;
+        if ((error = cudaMemPoolCreate(&made, &props)) != cudaSuccess) return error;
+        if ((error = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+            cudaMemPoolDestroy(made);
+            return error;
+        }
+        gWorkspacePool[device] = made;
+    }
+    *pool = gWorkspacePool[device];
+    return cudaSuccess;
+}
+
+// Device memory from the pool, in stream order (freed with cudaFreeAsync).
+template <class T>
+cudaError_t workspace(T** memory, size_t bytes, cudaStream_t stream) {
+    cudaMemPool_t pool = nullptr;
+    const cudaError_t error = workspacePool(&pool, true);
+    if (error != cudaSuccess) return error;
+    return cudaMallocFromPoolAsync(reinterpret_cast<void**>(memory), bytes, pool, stream);
+}
+
+void trimWorkspace() {
+    cudaMemPool_t pool = nullptr;
+    if (workspacePool(&pool, false) == cudaSuccess && pool) cudaMemPoolTrimTo(pool, 0);
+}
+
+// giveBack: the workspace pool's unused memory goes back first, so that it counts as free.
+int queryDevice(sadcs_gpu_device* device, bool giveBack = false) {
     int count = 0;
     cudaError_t error = cudaGetDeviceCount(&count);
     if (error != cudaSuccess || count == 0) {
@@ -367,6 +420,7 @@ int queryDevice(sadcs_gpu_device* device) {
         return SADCS_UNAVAILABLE;
     }
     size_t freeBytes = 0, totalBytes = 0;
+    if (giveBack) trimWorkspace();
     if ((error = cudaMemGetInfo(&freeBytes, &totalBytes)) != cudaSuccess) {
         setError("cudaMemGetInfo: %s", cudaGetErrorString(error));
         return SADCS_UNAVAILABLE;
@@ -405,6 +459,9 @@ int createContext(int64_t capacity, uint32_t texts, sadcs_gpu_context** out, boo
     }
     const bool carry = carryRoom && planCarry(static_cast<uint64_t>(capacity), texts);
     const size_t bytes = contextBytes(capacity, texts, carry);
+    if (static_cast<int64_t>(bytes) + kMemoryReserve > device.free_bytes) {
+        if (const int status = queryDevice(&device, true); status != SADCS_OK) return status;
+    }
     if (static_cast<int64_t>(bytes) + kMemoryReserve > device.free_bytes) {
         setError("needs %lld MiB of device memory plus %lld MiB reserve, %lld MiB free",
                  static_cast<long long>(bytes >> 20), static_cast<long long>(kMemoryReserve >> 20),
@@ -867,7 +924,7 @@ int64_t sadcs_gpu_sample_size(int64_t n) {
 
 int sadcs_gpu_query_device(sadcs_gpu_device* device) {
     tLastError[0] = '\0';
-    return queryDevice(device);
+    return queryDevice(device, true);
 }
 
 int64_t sadcs_gpu_required_bytes(int64_t n) {
@@ -1100,18 +1157,11 @@ int sadcs_gpu_bwt_from_sa(const uint8_t* d_text, int64_t n, const uint32_t* d_sa
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint32_t* word = nullptr;
-    uint32_t* host = nullptr;
     cudaError_t error;
-    if ((error = cudaMallocAsync(&word, sizeof(uint32_t), st)) != cudaSuccess) return failed("cudaMallocAsync", error);
-    if ((error = cudaMallocHost(&host, sizeof(uint32_t))) != cudaSuccess) {
-        cudaFreeAsync(word, st);
-        return failed("cudaMallocHost", error);
-    }
+    if ((error = workspace(&word, sizeof(uint32_t), st)) != cudaSuccess) return failed("allocating the gather's word", error);
     uint32_t row0 = 0;
-    error = bwtFromSa(d_text, static_cast<uint32_t>(n), d_sa, d_bwt, word, host, st, &row0);
+    error = bwtFromSa(d_text, static_cast<uint32_t>(n), d_sa, d_bwt, word, st, &row0);
     cudaFreeAsync(word, st);
-    cudaStreamSynchronize(st);
-    cudaFreeHost(host);
     if (error != cudaSuccess) return failed("SA-to-BWT gather", error);
     if (primary) *primary = static_cast<int64_t>(row0) + 1;
     return SADCS_OK;
@@ -1131,13 +1181,11 @@ int sadcs_gpu_check_suffix_array(const uint8_t* d_text, int64_t n, const uint32_
     const uint32_t count = static_cast<uint32_t>(n);
     uint32_t* isa = nullptr;
     unsigned long long* words = nullptr;
-    unsigned long long* host = nullptr;
+    unsigned long long host[3] = {kNoFailure, kNoFailure, kNoFailure};
     cudaError_t error;
-    if ((error = cudaMallocAsync(&isa, 4 * static_cast<size_t>(n), st)) != cudaSuccess) return failed("cudaMallocAsync", error);
-    if ((error = cudaMallocAsync(&words, 3 * sizeof(unsigned long long), st)) != cudaSuccess ||
-        (error = cudaMallocHost(&host, 3 * sizeof(unsigned long long))) != cudaSuccess) {
+    if ((error = workspace(&isa, 4 * static_cast<size_t>(n), st)) != cudaSuccess) return failed("allocating check buffers", error);
+    if ((error = workspace(&words, 3 * sizeof(unsigned long long), st)) != cudaSuccess) {
         cudaFreeAsync(isa, st);
-        if (words) cudaFreeAsync(words, st);
         return failed("allocating check buffers", error);
     }
     const uint32_t blocks = (count + 255) / 256;
@@ -1169,7 +1217,6 @@ int sadcs_gpu_check_suffix_array(const uint8_t* d_text, int64_t n, const uint32_
     cudaFreeAsync(isa, st);
     cudaFreeAsync(words, st);
     cudaStreamSynchronize(st);
-    cudaFreeHost(host);
     if (error != cudaSuccess) return failed("suffix array check", error);
     if (bad_index) *bad_index = index;
     if (reason) *reason = why;
@@ -1267,19 +1314,14 @@ namespace {
 // Inverse BWT into d_out with temporary device memory; valid = false for a broken BWT.
 int inverseWithScratch(const uint8_t* d_bwt, int64_t n, int64_t primary, uint8_t* d_out, cudaStream_t st, bool& valid) {
     uint32_t* scratch = nullptr;
-    uint32_t* host = nullptr;
+    uint32_t host[4] = {};
     cudaError_t error;
-    if ((error = cudaMallocAsync(&scratch, 4 * inverseScratchWords(static_cast<uint64_t>(n)), st)) != cudaSuccess) {
-        return failed("cudaMallocAsync", error);
-    }
-    if ((error = cudaMallocHost(&host, 16)) != cudaSuccess) {
-        cudaFreeAsync(scratch, st);
-        return failed("cudaMallocHost", error);
+    if ((error = workspace(&scratch, 4 * inverseScratchWords(static_cast<uint64_t>(n)), st)) != cudaSuccess) {
+        return failed("allocating the inverse's scratch", error);
     }
     error = inverseBwt(d_bwt, static_cast<uint32_t>(n), static_cast<uint32_t>(primary), d_out, scratch, host, st, valid);
     cudaFreeAsync(scratch, st);
     cudaStreamSynchronize(st);
-    cudaFreeHost(host);
     return error == cudaSuccess ? SADCS_OK : failed("inverse BWT", error);
 }
 
@@ -1322,10 +1364,10 @@ int sadcs_gpu_check_bwt(const uint8_t* d_text, int64_t n, const uint8_t* d_bwt, 
     unsigned long long* word = nullptr;
     unsigned long long host = 0;
     cudaError_t error;
-    if ((error = cudaMallocAsync(&inverse, static_cast<size_t>(n), st)) != cudaSuccess ||
-        (error = cudaMallocAsync(&word, 8, st)) != cudaSuccess) {
+    if ((error = workspace(&inverse, static_cast<size_t>(n), st)) != cudaSuccess ||
+        (error = workspace(&word, 8, st)) != cudaSuccess) {
         if (inverse) cudaFreeAsync(inverse, st);
-        return failed("cudaMallocAsync", error);
+        return failed("allocating check buffers", error);
     }
     bool valid = true;
     int status = inverseWithScratch(d_bwt, n, primary, inverse, st, valid);
@@ -1490,8 +1532,8 @@ int sadcs_gpu_lcp(const uint8_t* d_text, int64_t n, const uint32_t* d_sa, uint32
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     PhaseRange phase("sadcs lcp");
     uint32_t* scratch = nullptr;
-    cudaError_t error = cudaMallocAsync(&scratch, 4 * lcp::scratchWords(static_cast<uint64_t>(n)), st);
-    if (error != cudaSuccess) return failed("cudaMallocAsync", error);
+    cudaError_t error = workspace(&scratch, 4 * lcp::scratchWords(static_cast<uint64_t>(n)), st);
+    if (error != cudaSuccess) return failed("allocating the LCP scratch", error);
     error = lcp::lcpArray(d_text, static_cast<uint32_t>(n), d_sa, d_lcp, scratch, st);
     cudaFreeAsync(scratch, st);
     const cudaError_t done = cudaStreamSynchronize(st);

@@ -277,7 +277,7 @@ int sadcs_gpu_server_create(int64_t memory_budget, int32_t workers, int64_t smal
     }
     *out = nullptr;
     sadcs_gpu_device device;
-    if (const int status = queryDevice(&device); status != SADCS_OK) return status;
+    if (const int status = queryDevice(&device, true); status != SADCS_OK) return status;
     if (workers < 1 || workers > 64 || batch_texts < 1 || static_cast<uint32_t>(batch_texts) > kMaxTexts ||
         small_limit < 0 || batch_bytes < small_limit || batch_bytes > kMaxText) {
         setError("server parameters out of range");
