@@ -165,7 +165,8 @@ int sadcs_gpu_build_batch_device(sadcs_gpu_context* context, const uint8_t* d_te
 /* No counterpart: the reference checker's fast mode (src/common/checker.cpp:53-109) on the device.
  * Device buffers: d_text (n bytes), d_sa (n uint32 entries). *bad_index gets -1 if the suffix array
  * is correct, else the first failing SA index; *reason (if not NULL) a static description. Uses 4n
- * bytes of temporary device memory. Returns SADCS_OK whenever the check ran. */
+ * bytes of temporary device memory, and from 16M entries on 8n more where they are to be had. Returns
+ * SADCS_OK whenever the check ran. */
 int sadcs_gpu_check_suffix_array(const uint8_t* d_text, int64_t n, const uint32_t* d_sa, int64_t* bad_index,
                                  const char** reason, void* stream);
 
@@ -250,8 +251,8 @@ int sadcs_gpu_inverse_bwt(const uint8_t* d_bwt, int64_t n, int64_t primary, uint
  * array on the device. lcp[0] = 0 and lcp[r] = the length of the longest common prefix of suffixes
  * d_sa[r - 1] and d_sa[r], for d_sa (n uint32 entries) the suffix array of d_text (n bytes, no
  * padding needed), n up to 2^32 - 256. d_lcp gets n uint32 entries and may be d_sa itself (the
- * suffix array is then replaced by its LCP array). Uses about 4.13n bytes of temporary device memory;
- * returns when the array is complete. A d_sa that is not the suffix array of d_text gives an
+ * suffix array is then replaced by its LCP array). Uses about 4.13n bytes of temporary device memory,
+ * and from 16M entries on 8n more where they are to be had; returns when the array is complete. A d_sa that is not the suffix array of d_text gives an
  * unspecified d_lcp, never a read outside the buffers. */
 int sadcs_gpu_lcp(const uint8_t* d_text, int64_t n, const uint32_t* d_sa, uint32_t* d_lcp, void* stream);
 

@@ -56,6 +56,59 @@ __global__ void checkOrder(const uint8_t* __restrict__ text, const uint32_t* __r
     if (!ok) atomicMin(firstBad, static_cast<unsigned long long>(i));
 }
 
+// ---- the check of a correct suffix array ---------------------------------------------------------
+//
+// The same conditions, for the common case that they hold: no failing index is kept, so the inverse
+// suffix array needs no order among equal entries and is written slice by slice (scatterBySlices), and
+// one pass reads each entry's inverse once for both conditions. A suffix array that fails goes to the
+// kernels above, which find the first failing index. isa starts as all ones, which no entry is.
+struct InversePairs {
+    const uint32_t* __restrict__ sa;
+    uint32_t n;
+    __device__ __forceinline__ uint64_t operator()(uint32_t i) const {
+        const uint32_t p = __ldcs(sa + i);
+        return p < n ? (static_cast<uint64_t>(p) << 32) | i : kNoPair;
+    }
+};
+
+// failed != 0 unless every i has sa[i] < n, isa[sa[i]] = i (so sa is a permutation: n distinct slots are
+// owned), and neighbours in order by (first character, inverse of the suffix after it). Bound by its two
+// random reads per entry, isa[sa[i]] (with the entry after it, usually the same sector) and the
+// character: each is read once and handed to the entry before by the warp, the last lane's by
+// memory.
+constexpr int kVerifyThreads = 256;
+__global__ void __launch_bounds__(kVerifyThreads) checkVerify(const uint8_t* __restrict__ text,
+                                                              const uint32_t* __restrict__ sa, uint32_t n,
+                                                              const uint32_t* __restrict__ isa,
+                                                              uint32_t* __restrict__ failed) {
+    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kVerifyThreads + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31;
+    // (first character, 1 + inverse of the suffix after it, 0 for the empty one) of entry e; owned: isa says so too
+    const auto look = [&](uint64_t e, uint32_t& c, uint32_t& after, bool& owned) {
+        const uint32_t p = sa[e];
+        c = after = 0;
+        owned = p < n;
+        if (owned) {
+            owned = isa[p] == e;
+            c = text[p];
+            after = p + 1 < n ? isa[p + 1] + 1 : 0;
+        }
+    };
+    uint32_t c = 0, after = 0;
+    bool owned = true;
+    if (i < n) look(i, c, after, owned);
+    uint32_t c2 = __shfl_down_sync(0xffffffffu, c, 1), after2 = __shfl_down_sync(0xffffffffu, after, 1);
+    bool ok = owned;
+    if (i + 1 < n) {
+        if (lane == 31) {
+            bool owned2;
+            look(i + 1, c2, after2, owned2);
+        }
+        ok = ok && (c < c2 || (c == c2 && after < after2));
+    }
+    if (!ok) *failed = 1;
+}
+
 }  // namespace sadcs
 
 namespace sadcs {

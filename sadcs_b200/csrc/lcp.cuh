@@ -14,7 +14,8 @@
 //   with the reducible entries set to 0 gives V everywhere: PLCP[p] = scan(V)[p] - p.
 //   lcp[r] = PLCP[sa[r]].
 // Passes (one u32 scratch entry per position, Phi then V in place):
-//   lcpPhi      reads sa (coalesced, 8 B/entry), writes Phi at random (4 B/entry)
+//   lcpPhi      reads sa (coalesced, 8 B/entry), writes Phi at random (4 B/entry); large arrays by
+//               slices instead (scatterBySlices: pairs out and in, 8 B each, writes within L2)
 //   lcpShort    reads Phi, T[p - 1] (coalesced) and T[Phi[p] - 1] (random); at irreducible
 //               positions one thread compares up to kThreadBytes characters by 8-byte windows;
 //               writes V, and one bit per position marks comparisons left unfinished
@@ -164,6 +165,16 @@ __global__ void __launch_bounds__(kThreads) lcpPhi(const uint32_t* __restrict__ 
     if (r < n) phiAt(sa, n, static_cast<uint32_t>(r), phi);
 }
 
+// The same as pairs (position, Phi) for scatterBySlices.
+struct PhiPairs {
+    const uint32_t* __restrict__ sa;
+    uint32_t n;
+    __device__ __forceinline__ uint64_t operator()(uint32_t r) const {
+        const uint32_t p = sa[r];
+        return p < n ? (static_cast<uint64_t>(p) << 32) | (r ? sa[r - 1] : kNone) : kNoPair;
+    }
+};
+
 // One thread per position, a warp per 32 positions: the warp's ballot of unfinished comparisons is
 // word p / 32 of the mask (every word is written, none needs clearing).
 template <bool kAligned>
@@ -210,15 +221,26 @@ __global__ void __launch_bounds__(kThreads) lcpGather(const uint32_t* sa, const 
     if (r < n) out[r] = gatherAt(sa, v, n, static_cast<uint32_t>(r));
 }
 
-// Scratch words of lcpArray for n positions: Phi/V, the mask, the scan's scratch.
-inline size_t scratchWords(uint64_t n) {
-    return n + (ceilDiv(n, 32) + 63) / 64 * 64 + scanScratchWords(n);
+// Scratch words of lcpArray for n positions: Phi/V, the mask, the scan's scratch; with pairs, also
+// the pairs of the sliced Phi scatter.
+inline size_t scratchWords(uint64_t n, bool pairs = false) {
+    const size_t words = n + (ceilDiv(n, 32) + 63) / 64 * 64 + scanScratchWords(n);
+    return pairs ? words + words % 2 + 2 * n + kMaxSlices : words;
 }
 
+// Arrays past the L2's size take their Phi by slices: at 128 MiB 2.0 ms (partition and scatter)
+// against 5.35 ms for the one-pass scatter, whose every write is a sector of DRAM read and written;
+// below it the one pass writes L2 (tuning).
+#ifndef SADCS_SLICED_SCATTER_MIN
+#define SADCS_SLICED_SCATTER_MIN (16u << 20)
+#endif
+inline bool slicedScatter(uint64_t n) { return n >= SADCS_SLICED_SCATTER_MIN; }
+
 // The LCP array of sa (n entries, n <= 2^32 - 256) into out, on stream; out may be sa itself (each
-// entry is read before it is written, by the same thread). scratch: scratchWords(n) words.
+// entry is read before it is written, by the same thread). scratch: scratchWords(n, pairs) words; pairs:
+// Phi by slices.
 inline cudaError_t lcpArray(const uint8_t* text, uint32_t n, const uint32_t* sa, uint32_t* out, uint32_t* scratch,
-                            cudaStream_t stream) {
+                            bool pairs, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
     uint32_t* phiV = scratch;
     const uint32_t words = ceilDiv(n, 32);
@@ -227,7 +249,13 @@ inline cudaError_t lcpArray(const uint8_t* text, uint32_t n, const uint32_t* sa,
     const uint32_t blocks = ceilDiv(n, kThreads);
     const uint32_t longBlocks = std::min<uint32_t>(ceilDiv(words, kThreads / 32), 148u * 8);
     const bool aligned = (reinterpret_cast<uintptr_t>(text) & 7) == 0;
-    SADCS_TRY(launch(lcpPhi, blocks, kThreads, 0, stream, sa, n, phiV));
+    if (pairs) {
+        const size_t words = scratchWords(n) + scratchWords(n) % 2;
+        uint64_t* pairWords = reinterpret_cast<uint64_t*>(scratch + words);
+        SADCS_TRY(scatterBySlices(PhiPairs{sa, n}, n, phiV, pairWords, scratch + words + 2 * static_cast<size_t>(n), stream));
+    } else {
+        SADCS_TRY(launch(lcpPhi, blocks, kThreads, 0, stream, sa, n, phiV));
+    }
     if (aligned) {
         SADCS_TRY(launch(lcpShort<true>, blocks, kThreads, 0, stream, text, n, phiV, mask));
         SADCS_TRY(launch(lcpLong<true>, longBlocks, kThreads, 0, stream, text, n, mask, words, phiV));

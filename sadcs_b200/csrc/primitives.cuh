@@ -265,6 +265,70 @@ __device__ __forceinline__ void writeSliceMajor(SliceStage& st, const uint64_t (
     }
 }
 
+// Pairs source(0) .. source(count - 1) (kNoPair: none) -> dst, slice-major. fill[k] (zeroed by the
+// caller) counts the pairs placed in slice k.
+template <class Source>
+__global__ void __launch_bounds__(kSliceThreads) slicePartition(Source source, uint32_t count, uint32_t shift,
+                                                                uint32_t* __restrict__ fill,
+                                                                uint64_t* __restrict__ dst, uint64_t capacity) {
+    __shared__ SliceStage stage;
+    uint64_t v[kSliceItems];
+    const uint64_t first = static_cast<uint64_t>(blockIdx.x) * kSliceTile + threadIdx.x;
+#pragma unroll
+    for (int j = 0; j < kSliceItems; j++) {
+        const uint64_t i = first + static_cast<uint64_t>(j) * kSliceThreads;
+        v[j] = i < count ? source(static_cast<uint32_t>(i)) : kNoPair;
+        // no pair, or one whose index no slice holds
+        if ((static_cast<uint32_t>(v[j] >> 32) >> shift) >= kMaxSlices) v[j] = kNoPair;
+    }
+    writeSliceMajor(stage, v, shift, fill, dst, capacity);
+}
+
+// out[index] = value of every pair of the slice-major dst, the slices one after another, so that a
+// slice's writes stay within a part of out that L2 holds. Block b takes the pairs of
+// dst[b * kPairTile, (b + 1) * kPairTile) that its slice holds; limit: entries of out.
+constexpr int kPairThreads = 256;
+constexpr int kPairItems = 8;
+constexpr uint32_t kPairTile = kPairThreads * kPairItems;  // divides every slice
+__global__ void __launch_bounds__(kPairThreads) sliceScatter(const uint64_t* __restrict__ dst, uint32_t shift,
+                                                             uint64_t capacity, uint32_t limit,
+                                                             const uint32_t* __restrict__ fill,
+                                                             uint32_t* __restrict__ out) {
+    const uint64_t start = static_cast<uint64_t>(blockIdx.x) * kPairTile;
+    const uint32_t k = static_cast<uint32_t>(start >> shift);
+    const uint64_t end = min((static_cast<uint64_t>(k) << shift) + __ldg(fill + k), capacity);
+    for (uint64_t i = start + threadIdx.x; i < min(end, start + kPairTile); i += kPairThreads) {
+        const uint64_t v = __ldcs(dst + i);
+        const uint32_t t = static_cast<uint32_t>(v >> 32);
+        if (t < limit) out[t] = static_cast<uint32_t>(v);
+    }
+}
+
+// The slice width (as a shift) for a target of `entries` words: 4M words = 16 MB (at 3 GiB 0.6 ms
+// less ranking than 8M), more where that would give more than kMaxSlices slices.
+#ifndef SADCS_SLICE_SHIFT
+#define SADCS_SLICE_SHIFT 22
+#endif
+inline uint32_t sliceShift(uint64_t entries) {
+    uint32_t shift = SADCS_SLICE_SHIFT;
+    while ((entries >> shift) >= kMaxSlices) shift++;
+    return shift;
+}
+
+// out[index] = value for the pairs of source(0) .. source(n - 1), whose indices are distinct and below
+// n (of pairs that are not, some may be left out, and none leaves the buffers). pairs: n words;
+// fill: kMaxSlices words.
+template <class Source>
+cudaError_t scatterBySlices(const Source& source, uint32_t n, uint32_t* out, uint64_t* pairs, uint32_t* fill,
+                            cudaStream_t stream) {
+    const uint32_t shift = sliceShift(n);
+    SADCS_TRY(cudaMemsetAsync(fill, 0, kMaxSlices * sizeof(uint32_t), stream));
+    SADCS_TRY(launch(slicePartition<Source>, ceilDiv(n, kSliceTile), kSliceThreads, 0, stream, source, n, shift, fill,
+                     pairs, static_cast<uint64_t>(n)));
+    return launch(sliceScatter, ceilDiv(n, kPairTile), kPairThreads, 0, stream, pairs, shift, static_cast<uint64_t>(n),
+                  n, fill, out);
+}
+
 // ---- radix pass (onesweep) ------------------------------------------------------------------
 //
 // One stable counting pass on an 8-bit digit per kernel, reading and writing each element once

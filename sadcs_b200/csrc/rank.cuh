@@ -384,24 +384,10 @@ __global__ void __launch_bounds__(kRefineThreads) rankRefineApply(const uint32_t
 // (sample, rank) pairs in list order (rankRefineApply), rankPartitionPairs moves them into the
 // slice of the rank array they belong to (slice k: samples [k << shift, (k + 1) << shift); a pass
 // writes each sample at most once, so slice k of the pair array has room for all of its pairs),
-// and rankScatterPairs writes the slices one after another, each within an L2-sized part of the
+// and sliceScatter (primitives.cuh) writes the slices one after another, each within an L2-sized part of the
 // rank array.
-#ifndef SADCS_RANK_SLICE_SHIFT
-#define SADCS_RANK_SLICE_SHIFT 22  // 4M samples = 16 MB of the rank array per slice (tuning: 0.6 ms less ranking than 8M at 3 GiB)
-#endif
-constexpr uint32_t kRankSliceShift = SADCS_RANK_SLICE_SHIFT;
-constexpr uint32_t kMaxRankSlices = kMaxSlices;
-constexpr int kPairThreads = 256;
-constexpr int kPairItems = 8;
-constexpr uint32_t kPairTile = kPairThreads * kPairItems;  // divides 2^kRankSliceShift
 // Passes writing fewer ranks than this write them directly.
 constexpr uint32_t kBucketedRankWrites = 8u << 20;
-
-inline uint32_t rankSliceShift(uint64_t slots) {
-    uint32_t shift = kRankSliceShift;
-    while ((slots >> shift) >= kMaxRankSlices) shift++;
-    return shift;
-}
 
 // pairs[0, count) -> dst, slice-major (writeSliceMajor); count = u (every element wrote) or u less
 // the kept total. fill[k] (zeroed by the caller) counts the pairs placed in slice k.
@@ -419,24 +405,9 @@ __global__ void __launch_bounds__(kSliceThreads) rankPartitionPairs(const uint64
         const uint64_t i = first + static_cast<uint64_t>(j) * kSliceThreads;
         v[j] = i < total ? __ldcs(pairs + i) : kNoPair;
         // no pair, or a guarded out-of-range sample
-        if ((static_cast<uint32_t>(v[j] >> 32) >> shift) >= kMaxRankSlices) v[j] = kNoPair;
+        if ((static_cast<uint32_t>(v[j] >> 32) >> shift) >= kMaxSlices) v[j] = kNoPair;
     }
     writeSliceMajor(stage, v, shift, fill, dst, capacity);
-}
-
-// Block b writes the pairs of dst[b * kPairTile, (b + 1) * kPairTile) that its slice holds.
-__global__ void __launch_bounds__(kPairThreads) rankScatterPairs(const uint64_t* __restrict__ dst, uint32_t shift,
-                                                                 uint32_t capacity, uint32_t slots,
-                                                                 const uint32_t* __restrict__ fill,
-                                                                 uint32_t* __restrict__ ranks) {
-    const uint64_t start = static_cast<uint64_t>(blockIdx.x) * kPairTile;
-    const uint32_t k = static_cast<uint32_t>(start >> shift);
-    const uint64_t end = min((static_cast<uint64_t>(k) << shift) + __ldg(fill + k), static_cast<uint64_t>(capacity));
-    for (uint64_t i = start + threadIdx.x; i < min(end, start + kPairTile); i += kPairThreads) {
-        const uint64_t v = __ldcs(dst + i);
-        const uint32_t t = static_cast<uint32_t>(v >> 32);
-        if (t < slots) ranks[t] = static_cast<uint32_t>(v);
-    }
 }
 
 inline uint32_t blocks256(uint64_t count) {
@@ -559,13 +530,13 @@ inline cudaError_t rankSample(const uint8_t* text, const TextSet& texts, uint32_
                          b.aux1, ranks, lstAlt, b.aux2, writeAll ? 1u : 0u, bucketed ? keyAlt : nullptr));
         if (bucketed) {
             // the sorted keys are dead now: they become the slice-major pair array
-            const uint32_t shift = rankSliceShift(slots);
+            const uint32_t shift = sliceShift(slots);
             uint32_t* fill = b.scratch;  // the first sort's digit bases, dead after it
-            SADCS_TRY(cudaMemsetAsync(fill, 0, kMaxRankSlices * sizeof(uint32_t), stream));
+            SADCS_TRY(cudaMemsetAsync(fill, 0, kMaxSlices * sizeof(uint32_t), stream));
             SADCS_TRY(launch(rankPartitionPairs, ceilDiv(u, kSliceTile), kSliceThreads, 0, stream, keyAlt, u,
                              b.counter, writeAll ? 1u : 0u, shift, b.keyEntries, fill, key));
-            SADCS_TRY(launch(rankScatterPairs, ceilDiv(slots, kPairTile), kPairThreads, 0, stream, key, shift,
-                             b.keyEntries, slots, fill, ranks));
+            SADCS_TRY(launch(sliceScatter, ceilDiv(slots, kPairTile), kPairThreads, 0, stream, key, shift,
+                             static_cast<uint64_t>(b.keyEntries), slots, fill, ranks));
         }
         std::swap(b.grp, b.aux2);  // the kept elements' ids are the next pass's groups
         SADCS_TRY(cudaMemcpyAsync(hostCounter, b.counter, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));

@@ -1179,43 +1179,68 @@ int sadcs_gpu_check_suffix_array(const uint8_t* d_text, int64_t n, const uint32_
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const uint32_t count = static_cast<uint32_t>(n);
+    // The inverse suffix array, three result words (all ones: no failure) and, for arrays past the
+    // L2's size, the pairs of the sliced scatter, where there is memory for them.
     uint32_t* isa = nullptr;
     unsigned long long* words = nullptr;
+    uint64_t* pairs = nullptr;
     unsigned long long host[3] = {kNoFailure, kNoFailure, kNoFailure};
     cudaError_t error;
     if ((error = workspace(&isa, 4 * static_cast<size_t>(n), st)) != cudaSuccess) return failed("allocating check buffers", error);
-    if ((error = workspace(&words, 3 * sizeof(unsigned long long), st)) != cudaSuccess) {
+    if ((error = workspace(&words, 4 * sizeof(unsigned long long), st)) != cudaSuccess) {
         cudaFreeAsync(isa, st);
         return failed("allocating check buffers", error);
     }
+    if (lcp::slicedScatter(static_cast<uint64_t>(n)) &&
+        workspace(&pairs, 8 * static_cast<size_t>(n) + 4 * kMaxSlices, st) != cudaSuccess) {
+        cudaGetLastError();
+        pairs = nullptr;
+    }
     const uint32_t blocks = (count + 255) / 256;
-    error = cudaMemsetAsync(words, 0xFF, 3 * sizeof(unsigned long long), st);
-    if (error == cudaSuccess) error = cudaMemsetAsync(isa, 0, 4 * static_cast<size_t>(count), st);
-    if (error == cudaSuccess) error = launch(checkScatter, blocks, 256, 0, st, d_sa, count, isa, words);
-    if (error == cudaSuccess) error = cudaMemcpyAsync(host, words, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
+    uint32_t* failedWord = reinterpret_cast<uint32_t*>(words + 3);
+    uint32_t hostFailed = 0;
+    error = cudaMemsetAsync(failedWord, 0, sizeof(uint32_t), st);
+    if (error == cudaSuccess) error = cudaMemsetAsync(words, 0xFF, 3 * sizeof(unsigned long long), st);
+    if (error == cudaSuccess) error = cudaMemsetAsync(isa, pairs ? 0xFF : 0, 4 * static_cast<size_t>(count), st);
+    if (error == cudaSuccess) {
+        error = pairs ? scatterBySlices(InversePairs{d_sa, count}, count, isa, pairs,
+                                        reinterpret_cast<uint32_t*>(pairs + count), st)
+                      : launch(checkScatter, blocks, 256, 0, st, d_sa, count, isa, words);
+    }
+    if (error == cudaSuccess) error = launch(checkVerify, ceilDiv(count, kVerifyThreads), kVerifyThreads, 0, st, d_text, d_sa, count, isa, failedWord);
+    if (error == cudaSuccess) error = cudaMemcpyAsync(&hostFailed, failedWord, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
     if (error == cudaSuccess) error = cudaStreamSynchronize(st);
     const char* why = nullptr;
     int64_t index = -1;
-    if (error == cudaSuccess && host[0] != kNoFailure) {
-        why = "entry out of range";
-        index = static_cast<int64_t>(host[0]);
-    }
-    if (error == cudaSuccess && !why) {
-        error = launch(checkDuplicates, blocks, 256, 0, st, d_sa, count, isa, words + 1);
-        if (error == cudaSuccess) error = launch(checkOrder, blocks, 256, 0, st, d_text, d_sa, count, isa, words + 2);
-        if (error == cudaSuccess)
-            error = cudaMemcpyAsync(host + 1, words + 1, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
+    if (error == cudaSuccess && hostFailed) {  // the first failing index, and of what
+        if (pairs) {
+            error = cudaMemsetAsync(isa, 0, 4 * static_cast<size_t>(count), st);
+            if (error == cudaSuccess) error = launch(checkScatter, blocks, 256, 0, st, d_sa, count, isa, words);
+        }
+        if (error == cudaSuccess) error = cudaMemcpyAsync(host, words, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
         if (error == cudaSuccess) error = cudaStreamSynchronize(st);
-        if (error == cudaSuccess && host[1] != kNoFailure) {
-            why = "duplicate entry";
-            index = static_cast<int64_t>(host[1]);
-        } else if (error == cudaSuccess && host[2] != kNoFailure) {
-            why = "SA[index] and SA[index + 1] out of order";
-            index = static_cast<int64_t>(host[2]);
+        if (error == cudaSuccess && host[0] != kNoFailure) {
+            why = "entry out of range";
+            index = static_cast<int64_t>(host[0]);
+        }
+        if (error == cudaSuccess && !why) {
+            error = launch(checkDuplicates, blocks, 256, 0, st, d_sa, count, isa, words + 1);
+            if (error == cudaSuccess) error = launch(checkOrder, blocks, 256, 0, st, d_text, d_sa, count, isa, words + 2);
+            if (error == cudaSuccess)
+                error = cudaMemcpyAsync(host + 1, words + 1, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
+            if (error == cudaSuccess) error = cudaStreamSynchronize(st);
+            if (error == cudaSuccess && host[1] != kNoFailure) {
+                why = "duplicate entry";
+                index = static_cast<int64_t>(host[1]);
+            } else if (error == cudaSuccess && host[2] != kNoFailure) {
+                why = "SA[index] and SA[index + 1] out of order";
+                index = static_cast<int64_t>(host[2]);
+            }
         }
     }
     cudaFreeAsync(isa, st);
     cudaFreeAsync(words, st);
+    if (pairs) cudaFreeAsync(pairs, st);
     cudaStreamSynchronize(st);
     if (error != cudaSuccess) return failed("suffix array check", error);
     if (bad_index) *bad_index = index;
@@ -1532,9 +1557,16 @@ int sadcs_gpu_lcp(const uint8_t* d_text, int64_t n, const uint32_t* d_sa, uint32
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     PhaseRange phase("sadcs lcp");
     uint32_t* scratch = nullptr;
-    cudaError_t error = workspace(&scratch, 4 * lcp::scratchWords(static_cast<uint64_t>(n)), st);
+    const uint64_t count = static_cast<uint64_t>(n);
+    bool pairs = lcp::slicedScatter(count);
+    cudaError_t error = workspace(&scratch, 4 * lcp::scratchWords(count, pairs), st);
+    if (error != cudaSuccess && pairs) {  // no memory for the pairs: Phi in one pass
+        cudaGetLastError();
+        pairs = false;
+        error = workspace(&scratch, 4 * lcp::scratchWords(count), st);
+    }
     if (error != cudaSuccess) return failed("allocating the LCP scratch", error);
-    error = lcp::lcpArray(d_text, static_cast<uint32_t>(n), d_sa, d_lcp, scratch, st);
+    error = lcp::lcpArray(d_text, static_cast<uint32_t>(n), d_sa, d_lcp, scratch, pairs, st);
     cudaFreeAsync(scratch, st);
     const cudaError_t done = cudaStreamSynchronize(st);
     if (error == cudaSuccess) error = done;

@@ -1,0 +1,61 @@
+"""The suffix array check's fast path (sliced inverse, one pass) and its hand-over to the kernels that
+name the first failing index, on both sides of the size where the inverse is written by slices, and
+the LCP array there: verdict, index and reason as the one-pass kernels give them."""
+import numpy as np
+import pytest
+
+import sadcs_b200 as sa
+
+pytestmark = pytest.mark.gpu
+
+SLICED = 16 << 20  # entries from which arrays are written by slices
+
+
+def _lcp_of_neighbours(text, suffixes, limit=64):
+    """LCPs of neighbouring suffixes that are below `limit`, by comparing character by character."""
+    import torch
+
+    n = text.numel()
+    a, b = suffixes[:-1], suffixes[1:]
+    out = torch.zeros(n, dtype=torch.int64, device="cuda")
+    open_ = torch.ones(n - 1, dtype=torch.bool, device="cuda")
+    for k in range(limit):
+        inside = (a + k < n) & (b + k < n)
+        open_ &= inside & (text[(a + k).clamp(max=n - 1)] == text[(b + k).clamp(max=n - 1)])
+        out[1:] += open_
+    return out
+
+
+@pytest.mark.parametrize("n", [257, 100_000, SLICED - 1, SLICED, SLICED + 4097])
+def test_verdicts(n):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    text = torch.randint(0, 7, (n,), dtype=torch.uint8, device="cuda", generator=g)
+    suffixes = torch.empty(n, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    sa.build_device(text.data_ptr(), n, suffixes.data_ptr(), None)
+
+    def check():
+        torch.cuda.synchronize()
+        return sa.check_suffix_array_device(text.data_ptr(), n, suffixes.data_ptr())
+
+    assert check() == (True, -1, None)
+    lcp = torch.empty_like(suffixes)
+    sa.lcp_device(text.data_ptr(), n, suffixes.data_ptr(), lcp.data_ptr())
+    assert torch.equal(lcp.to(torch.int64), _lcp_of_neighbours(text, suffixes.to(torch.int64)))
+    correct = suffixes.clone()
+    i, j = n // 3, n - 2
+    suffixes[[i, i + 1]] = correct[[i + 1, i]]  # neighbours exchanged: the pair itself or one beside it
+    ok, index, reason = check()
+    assert not ok and index in (i - 1, i) and reason == "SA[index] and SA[index + 1] out of order"
+    suffixes.copy_(correct)
+    suffixes[j] = correct[i]  # the earlier of two equal entries is reported
+    assert check() == (False, i, "duplicate entry")
+    suffixes.copy_(correct)
+    suffixes[31] = n
+    suffixes[j] = n + 5
+    assert check() == (False, 31, "entry out of range")
+    suffixes.copy_(correct)
+    suffixes[0], suffixes[n - 1] = correct[n - 1], correct[0]
+    assert not check()[0]
