@@ -386,8 +386,10 @@ __global__ void __launch_bounds__(kRefineThreads) rankRefineApply(const uint32_t
 // writes each sample at most once, so slice k of the pair array has room for all of its pairs),
 // and sliceScatter (primitives.cuh) writes the slices one after another, each within an L2-sized part of the
 // rank array.
-// Passes writing fewer ranks than this write them directly.
+// Passes writing fewer ranks than this, or to an array that L2 holds, write them directly (48 MiB text
+// of long repeats, 11M samples: partition and scatter of its 14 large passes 1.47 ms).
 constexpr uint32_t kBucketedRankWrites = 8u << 20;
+constexpr uint32_t kBucketedRankSlots = 16u << 20;
 
 // pairs[0, count) -> dst, slice-major (writeSliceMajor); count = u (every element wrote) or u less
 // the kept total. fill[k] (zeroed by the caller) counts the pairs placed in slice k.
@@ -525,7 +527,7 @@ inline cudaError_t rankSample(const uint8_t* text, const TextSet& texts, uint32_
         SADCS_TRY(launch(rankRefineReduce, refineTiles, kRefineThreads, 0, stream, b.grp, key, u, refineTiles, b.aux1));
         SADCS_TRY(launch(rankRefineScan, 1, 256, 0, stream, b.aux1, refineTiles, b.counter));
         // A large pass writes its ranks through pairs in the free key buffer (bucketed, below).
-        const bool bucketed = u >= kBucketedRankWrites && slots <= b.keyEntries;
+        const bool bucketed = u >= kBucketedRankWrites && slots >= kBucketedRankSlots && slots <= b.keyEntries;
         SADCS_TRY(launch(rankRefineApply, refineTiles, kRefineThreads, 0, stream, b.grp, key, lst, u, slots, refineTiles,
                          b.aux1, ranks, lstAlt, b.aux2, writeAll ? 1u : 0u, bucketed ? keyAlt : nullptr));
         if (bucketed) {

@@ -36,7 +36,8 @@ constexpr uint32_t kSegCap = kSegChunk + kSegSmall;  // elements a block can hol
 constexpr int kSegThreads = 256;
 constexpr int kSegWarps = kSegThreads / 32;
 constexpr int kSegItems = kSegCap / kSegThreads;     // 8 at the default
-constexpr uint32_t kSegMaxLocal = kSegChunk;         // segments starting in a chunk (each has >= 1 element)
+constexpr uint32_t kSegMaxLocal = kSegChunk / (kSegTiny + 1) + 1;  // segments of kSegTiny + 1 on starting in a chunk
+static_assert(kSegMaxLocal <= 256, "one digit for a block's segments");
 
 // The segments' big-path tables (host-sized): begin, size and first tile of each big segment.
 struct ListSegments {
@@ -196,21 +197,28 @@ __global__ void segCopyBack(ListSegments segs, const uint64_t* __restrict__ kFro
     }
 }
 
-// The small segments starting in [blockIdx.x * kSegChunk, + kSegChunk): sorted by subkey in
-// shared memory and written to out (which may be in). keyBits: significant key bits.
+// The segments of kSegTiny + 1 to kSegSmall elements starting in [blockIdx.x * kSegChunk, + kSegChunk):
+// sorted by (segment, subkey) in shared memory, stable 8-bit passes, and written to out (which may
+// be in). Bound by the passes' barriers and serial warp matches, so: digits on which every segment's
+// keys agree have no pass (after a few doubling rounds the ranks of a group's members at p + h are close
+// together: 1-2 of 3 digits differ), the segments need one pass (none for a single one), and the
+// elements are spread evenly over the warps. The ranking of a 48 MiB text of versions of one document
+// took 16.7 ms with every pass made over the block's first warps, 13.6 now (of it 1.5 by the direct
+// rank writes of small arrays), of 256 MiB of natural-language-like text 17.8 and 16.9.
 __global__ void __launch_bounds__(kSegThreads, SADCS_SEGSORT_BLOCKS) segSortSmall(const uint32_t* __restrict__ heads, uint32_t segments,
                                                             const uint64_t* keyIn, const uint32_t* valIn,
                                                             uint64_t* keyOut, uint32_t* valOut, int keyBits) {
     extern __shared__ __align__(16) unsigned char smem[];
     uint64_t* sKey = reinterpret_cast<uint64_t*>(smem);                 // kSegCap
     uint32_t* sVal = reinterpret_cast<uint32_t*>(sKey + kSegCap);       // kSegCap
-    uint16_t* sSeg = reinterpret_cast<uint16_t*>(sVal + kSegCap);       // kSegCap
-    uint32_t* segStart = reinterpret_cast<uint32_t*>(sSeg + kSegCap);   // kSegMaxLocal + 1 (global start)
+    uint32_t* segStart = sVal + kSegCap;                                // kSegMaxLocal + 1 (global start)
     uint32_t* segLocal = segStart + kSegMaxLocal + 1;                   // kSegMaxLocal + 1 (local start)
     uint32_t* warpCount = segLocal + kSegMaxLocal + 1;                  // kSegWarps * 256
     uint32_t* digitStart = warpCount + kSegWarps * 256;                 // 256
+    uint8_t* sSeg = reinterpret_cast<uint8_t*>(digitStart + 256);       // kSegCap
     __shared__ uint32_t warpTotals[32];
-    __shared__ uint32_t sFirst, sCount, sTotal;
+    __shared__ uint32_t sFirst, sCount;
+    __shared__ uint32_t sDiffer[2];  // key bits (low, high) in which some segment's keys differ
 
     if (threadIdx.x == 0) {
         const uint32_t lo = blockIdx.x * kSegChunk, hi = lo + kSegChunk;
@@ -226,71 +234,82 @@ __global__ void __launch_bounds__(kSegThreads, SADCS_SEGSORT_BLOCKS) segSortSmal
         }
         sFirst = a;
         sCount = c - a;
+        sDiffer[0] = sDiffer[1] = 0;
     }
     __syncthreads();
-    const uint32_t first = sFirst, count = sCount;
-    // Local starts of the small segments (big ones get size 0 here).
+    const uint32_t first = sFirst, started = sCount;
+    // The block's segments in order: their starts in the list and in the block (their number in the
+    // high half of the scanned words, their elements in the low half: at most kSegCap).
+    static_assert(kSegCap < 65536, "elements in the low half");
     uint32_t running = 0;
-    for (uint32_t base = 0; base < count; base += kSegThreads) {
+    for (uint32_t base = 0; base < started; base += kSegThreads) {
         const uint32_t s = base + threadIdx.x;
-        uint32_t size = 0;
-        if (s < count) {
-            const uint32_t start = heads[first + s], end = heads[first + s + 1];
-            size = end - start <= kSegSmall && end - start > kSegTiny ? end - start : 0;  // tiny ones: segSortTiny
-            segStart[s] = start;
+        uint32_t size = 0, start = 0;
+        if (s < started) {
+            start = heads[first + s];
+            size = heads[first + s + 1] - start;
+            if (size > kSegSmall || size <= kSegTiny) size = 0;  // larger: onesweep passes; smaller: segSortTiny
         }
-        uint32_t total;
-        const uint32_t inclusive = blockInclusiveScan<OpSum>(size, warpTotals, total);
-        if (s < count) segLocal[s] = running + inclusive - size;
-        running += total;
-        __syncthreads();
+        const uint32_t mine = size ? (1u << 16) | size : 0;
+        uint32_t all;
+        const uint32_t before = running + blockInclusiveScan<OpSum>(mine, warpTotals, all) - mine;
+        if (size) {
+            segStart[before >> 16] = start;
+            segLocal[before >> 16] = before & 0xFFFF;
+        }
+        running += all;
     }
-    if (threadIdx.x == 0) {
-        segLocal[count] = running;
-        sTotal = running;
-    }
-    __syncthreads();
-    const uint32_t total = sTotal;
+    const uint32_t count = running >> 16, total = running & 0xFFFF;
     if (total == 0) return;
+    if (threadIdx.x == 0) segLocal[count] = total;
+    __syncthreads();
 
-    // Load: item j of warp w is element w * (kSegItems * 32) + j * 32 + lane, in segment order.
+    // Load: item j of warp w is element (w * per + j) * 32 + lane, in segment order.
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int per = static_cast<int>((total + kSegThreads - 1) / kSegThreads);  // at most kSegItems
+    const uint32_t warpBase = warp * per * 32 + lane;
     uint64_t key[kSegItems];
     uint32_t val[kSegItems];
     uint32_t seg[kSegItems];
+    uint64_t differ = 0;
 #pragma unroll
     for (int j = 0; j < kSegItems; j++) {
-        const uint32_t t = warp * (kSegItems * 32) + j * 32 + lane;
+        const uint32_t t = warpBase + j * 32;
         seg[j] = 0xFFFF;
-        if (t < total) {
-            uint32_t a = 0, b = count;  // last s with segLocal[s] <= t among the nonempty ones
+        if (j < per && t < total) {
+            uint32_t a = 0, b = count;  // last s with segLocal[s] <= t
             while (b - a > 1) {
                 const uint32_t mid = (a + b) >> 1;
                 if (segLocal[mid] <= t) a = mid; else b = mid;
             }
-            while (segLocal[a + 1] <= t) a++;  // skip empty (big) segments sharing the start
             const uint32_t g = segStart[a] + (t - segLocal[a]);
             key[j] = keyIn[g];
             val[j] = valIn[g];
             seg[j] = a;
+            differ |= key[j] ^ keyIn[segStart[a]];
         }
     }
-    int segBits = 0;
-    while ((1u << segBits) < count) segBits++;
-    const int keyPasses = (keyBits + 7) / 8, segPasses = (segBits + 7) / 8;
+    const uint32_t low = __reduce_or_sync(0xffffffffu, static_cast<uint32_t>(differ));
+    const uint32_t high = __reduce_or_sync(0xffffffffu, static_cast<uint32_t>(differ >> 32));
+    if (lane == 0) {
+        if (low) atomicOr(&sDiffer[0], low);
+        if (high) atomicOr(&sDiffer[1], high);
+    }
+    __syncthreads();
+    differ = (static_cast<uint64_t>(sDiffer[1]) << 32) | sDiffer[0];
     const uint32_t lt = (1u << lane) - 1;
-    for (int pass = 0; pass < keyPasses + segPasses; pass++) {
+    const int keyPasses = (keyBits + 7) / 8;
+    for (int pass = 0; pass <= keyPasses; pass++) {  // the last one by segment
+        if (pass < keyPasses ? ((differ >> (8 * pass)) & 0xFF) == 0 : count == 1) continue;
         for (int i = threadIdx.x; i < kSegWarps * 256; i += kSegThreads) warpCount[i] = 0;
         __syncthreads();
         uint32_t* myCount = warpCount + warp * 256;
         uint32_t rankDigit[kSegItems];
 #pragma unroll
         for (int j = 0; j < kSegItems; j++) {
+            if (j >= per) break;  // the same for the block
             uint32_t d = kNoDigit;
-            if (seg[j] != 0xFFFF) {
-                d = pass < keyPasses ? static_cast<uint32_t>(key[j] >> (8 * pass)) & 0xFF
-                                     : (seg[j] >> (8 * (pass - keyPasses))) & 0xFF;
-            }
+            if (seg[j] != 0xFFFF) d = pass < keyPasses ? static_cast<uint32_t>(key[j] >> (8 * pass)) & 0xFF : seg[j];
             const uint32_t peers = __match_any_sync(0xffffffffu, d);
             uint32_t before = 0;
             if (d != kNoDigit) before = myCount[d];
@@ -314,24 +333,24 @@ __global__ void __launch_bounds__(kSegThreads, SADCS_SEGSORT_BLOCKS) segSortSmal
         __syncthreads();
 #pragma unroll
         for (int j = 0; j < kSegItems; j++) {
+            if (j >= per) break;
             const uint32_t d = rankDigit[j] & 0x1FF;
             if (d != kNoDigit) {
                 const uint32_t pos = digitStart[d] + warpCount[warp * 256 + d] + (rankDigit[j] >> 9);
                 sKey[pos] = key[j];
                 sVal[pos] = val[j];
-                sSeg[pos] = static_cast<uint16_t>(seg[j]);
+                sSeg[pos] = static_cast<uint8_t>(seg[j]);
             }
         }
         __syncthreads();
 #pragma unroll
         for (int j = 0; j < kSegItems; j++) {
-            const uint32_t t = warp * (kSegItems * 32) + j * 32 + lane;
+            if (j >= per) break;
+            const uint32_t t = warpBase + j * 32;
             if (t < total) {
                 key[j] = sKey[t];
                 val[j] = sVal[t];
                 seg[j] = sSeg[t];
-            } else {
-                seg[j] = 0xFFFF;
             }
         }
         __syncthreads();
@@ -339,8 +358,8 @@ __global__ void __launch_bounds__(kSegThreads, SADCS_SEGSORT_BLOCKS) segSortSmal
     // Sorted by (segment, key): segment s occupies [segLocal[s], segLocal[s + 1]) again.
 #pragma unroll
     for (int j = 0; j < kSegItems; j++) {
-        const uint32_t t = warp * (kSegItems * 32) + j * 32 + lane;
-        if (t < total) {
+        const uint32_t t = warpBase + j * 32;
+        if (j < per && t < total) {
             const uint32_t s = seg[j];
             const uint32_t g = segStart[s] + (t - segLocal[s]);
             keyOut[g] = key[j];
@@ -350,7 +369,7 @@ __global__ void __launch_bounds__(kSegThreads, SADCS_SEGSORT_BLOCKS) segSortSmal
 }
 
 constexpr size_t segSortSharedBytes() {
-    return kSegCap * (8 + 4 + 2) + 2 * (kSegMaxLocal + 1) * 4 + (kSegWarps * 256 + 256) * 4 + 64;
+    return kSegCap * (8 + 4 + 1) + 2 * (kSegMaxLocal + 1) * 4 + (kSegWarps * 256 + 256) * 4 + 64;
 }
 
 // Scratch words of segmentedSort for a list of u elements (besides the list buffers and aux arrays).
