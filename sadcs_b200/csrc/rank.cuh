@@ -79,6 +79,7 @@ struct FirstKeys {
 
 struct FirstKeyLoader {
     FirstKeys keys;
+    const uint32_t* vote;
     __device__ __forceinline__ bool load(uint32_t, uint32_t i, uint32_t, uint64_t& k, uint32_t& d) const {
         k = keys(i);
         d = static_cast<uint32_t>(k) & 0xFF;
@@ -88,8 +89,8 @@ struct FirstKeyLoader {
 };
 
 // Stable LSD sort of samples [0, count) of one text by their first keyChars characters (the
-// ranking's first pass): as radixSortPairs, with the first pass's keys and values made by
-// FirstKeyLoader. On return keys/vals point at the sorted keys and sample indices.
+// ranking's first pass): one histogram pass for every digit, then one onesweep pass each, the first
+// with keys and values made by FirstKeyLoader. On return keys/vals point at the sorted keys and sample indices.
 inline cudaError_t rankFirstSort(const TextSet& texts, uint32_t count, int keyBits, uint64_t*& keys,
                                  uint64_t*& keysAlt, uint32_t*& vals, uint32_t*& valsAlt, uint32_t* scratchWords,
                                  cudaStream_t stream) {
@@ -100,14 +101,14 @@ inline cudaError_t rankFirstSort(const TextSet& texts, uint32_t count, int keyBi
     const uint32_t histBlocks = std::min<uint32_t>(ceilDiv(count, 256 * 16), 148 * 8);
     SADCS_TRY(launch(radixHistogramFrom<FirstKeys>, histBlocks, 256, 0, stream, FirstKeys{texts}, count, 0, passes,
                      scratch.digitBase));
-    SADCS_TRY(launch(radixDigitBase, passes, 256, 0, stream, scratch.digitBase));
+    SADCS_TRY(launch(radixDigitBase, passes, 256, 0, stream, scratch.digitBase, scratch.control + 8));
     for (int p = 0; p < passes; p++) {
         const SortStorer<uint64_t> st{keysAlt, valsAlt, count};
         if (p == 0) {
-            SADCS_TRY((radixOnesweepPass<uint64_t>(FirstKeyLoader{FirstKeys{texts}}, st, OneSegment{count}, count,
+            SADCS_TRY((radixOnesweepPass<uint64_t>(FirstKeyLoader{FirstKeys{texts}, scratch.control + 8}, st, OneSegment{count}, count,
                                                    ceilDiv(count, kSortTile), scratch.digitBase, scratch, stream)));
         } else {
-            const SortLoader<uint64_t> ld{keys, vals, 8 * p};
+            const SortLoader<uint64_t> ld{keys, vals, 8 * p, scratch.control + 8 + p};
             SADCS_TRY((radixOnesweepPass<uint64_t>(ld, st, OneSegment{count}, count, ceilDiv(count, kSortTile),
                                                    scratch.digitBase + p * 256, scratch, stream)));
         }
