@@ -38,7 +38,8 @@ struct RankBuffers {
     uint32_t* aux2;
     uint32_t* scratch;      // radix scratch words (radixScratchWords(m))
     uint32_t* scanScratch;  // scan scratch words (scanScratchWords(m))
-    uint32_t* segScratch;   // segmented-sort scratch (segScratchWords(m))
+    uint32_t* segScratch;   // segmented-sort scratch
+    size_t segWords;        // its words (segScratchWords(m))
     uint32_t* counter;      // device words: [0] list count, [4..7] segmented sort
     uint32_t keyEntries;    // 64-bit entries of each key buffer (the pair arrays of a bucketed rank write)
 };
@@ -518,7 +519,7 @@ inline cudaError_t rankSample(const uint8_t* text, const TextSet& texts, uint32_
             if (depth == 0) {
                 SADCS_TRY(launch(rankGatherGroups, blocks256(u), 256, 0, stream, ranks, lst, b.grp, u, slots));
             }
-            SegBuffers sb{error - 1, b.aux1, b.aux2, reinterpret_cast<uint32_t*>(keyAlt), b.segScratch,
+            SegBuffers sb{error - 1, b.aux1, b.aux2, reinterpret_cast<uint32_t*>(keyAlt), b.segScratch, b.segWords,
                           b.counter + 4, b.scanScratch};
             SADCS_TRY(segmentedSort(b.grp, u, key, lst, keyAlt, lstAlt, keyBits, sb, hostCounter + 8, stream));
         }
