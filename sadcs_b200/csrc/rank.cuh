@@ -464,13 +464,15 @@ constexpr uint64_t kDeepChars = 20;
 struct RankStats {
     int characterPasses = 0;
     int doublingRounds = 0;
-    uint64_t deep = 0;  // samples that shared their first kDeepChars characters or more with another
+    // Samples that shared about kDeepChars characters or more with another: those still listed after the
+    // pass that reached them and those compared directly until then.
+    uint64_t deep = 0;
 };
 
 // Ranks the live sample suffixes of the texts. slots = rank entries (sample positions of the whole
 // concatenation); live = live samples; sampleBase (device, per text) is used with several texts.
 // Ranks of live samples end up in [0, live), text by text; ranks are zeroed by the caller for one
-// text (and kRankPad entries past slots always). hostCounter: two page-locked words.
+// text (and kRankPad entries past slots always). hostCounter: page-locked words (11).
 inline cudaError_t rankSample(const uint8_t* text, const TextSet& texts, uint32_t slots, uint32_t live,
                               const uint32_t* sampleBase, uint32_t longest, uint32_t* ranks, RankBuffers b,
                               uint32_t* hostCounter, cudaStream_t stream, RankStats& stats) {
@@ -483,7 +485,8 @@ inline cudaError_t rankSample(const uint8_t* text, const TextSet& texts, uint32_
     uint32_t* error = radixErrorWord(b.scratch);
     SADCS_TRY(cudaMemsetAsync(error, 0, sizeof(uint32_t), stream));
     uint32_t u = live;
-    uint64_t depth = 0;
+    uint64_t depth = 0, direct = 0;
+    bool deepKnown = false;
     bool first = texts.count <= 1;  // one text: everything starts in one group, no group sort
     const int rankBits = bitWidth(static_cast<uint64_t>(live) + 1);
     // The first pass of one text may key fewer characters (fewer radix passes over every sample).
@@ -502,6 +505,7 @@ inline cudaError_t rankSample(const uint8_t* text, const TextSet& texts, uint32_
         uint64_t* key = b.key[0];
         uint64_t* keyAlt = b.key[1];
         const TextSet& passTexts = first ? firstTexts : texts;
+        bool compared = false;
         if (!first) {
             SADCS_TRY(launch(rankMakeKeys, blocks256(u), 256, 0, stream, text, ranks, passTexts, lst, key, u, offset,
                              doubling ? 1 : 0));
@@ -520,8 +524,11 @@ inline cudaError_t rankSample(const uint8_t* text, const TextSet& texts, uint32_
                 SADCS_TRY(launch(rankGatherGroups, blocks256(u), 256, 0, stream, ranks, lst, b.grp, u, slots));
             }
             SegBuffers sb{error - 1, b.aux1, b.aux2, reinterpret_cast<uint32_t*>(keyAlt), b.segScratch, b.segWords,
-                          b.counter + 4, b.scanScratch};
-            SADCS_TRY(segmentedSort(b.grp, u, key, lst, keyAlt, lstAlt, keyBits, sb, hostCounter + 8, stream));
+                          b.counter + 4, b.scanScratch, &compared};
+            const uint64_t shared = depth + (doubling ? offset : passTexts.keyChars);  // by elements of equal keys
+            SADCS_TRY(segmentedSort(b.grp, u, key, lst, keyAlt, lstAlt, keyBits, texts,
+                                    static_cast<uint32_t>(std::min<uint64_t>(shared, 0xFFFFFFFFu)), sb,
+                                    hostCounter + 8, stream));
         }
         // The next pass reads ranks of other samples when it is a doubling round.
         const bool writeAll = doubling || depth + passTexts.keyChars >= kV;
@@ -545,6 +552,7 @@ inline cudaError_t rankSample(const uint8_t* text, const TextSet& texts, uint32_
         std::swap(b.grp, b.aux2);  // the kept elements' ids are the next pass's groups
         SADCS_TRY(cudaMemcpyAsync(hostCounter, b.counter, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
         SADCS_TRY(cudaMemcpyAsync(hostCounter + 1, error, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
+        if (compared) SADCS_TRY(cudaMemcpyAsync(hostCounter + 2, b.counter + 7, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
         SADCS_TRY(cudaStreamSynchronize(stream));
         if (hostCounter[1]) return cudaErrorLaunchTimeout;  // a radix look-back gave up
         if (traceEnabled()) {
@@ -561,7 +569,11 @@ inline cudaError_t rankSample(const uint8_t* text, const TextSet& texts, uint32_
             stats.characterPasses++;
             depth += passTexts.keyChars;
         }
-        if (depth >= kDeepChars && stats.deep == 0) stats.deep = u;
+        if (!deepKnown) {
+            if (compared) direct += hostCounter[2];
+            stats.deep = u + direct;
+            deepKnown = depth >= kDeepChars;
+        }
         first = false;
     }
     return cudaSuccess;

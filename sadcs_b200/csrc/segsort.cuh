@@ -5,7 +5,8 @@
 // Most segments are small (on genome-like text every segment left after the first pass has at most
 // 4 members; on natural-language text 80-95% of the remaining suffixes are in segments of up to a
 // few thousand), so:
-//   - segments of up to kSegTiny elements are sorted by one thread each in registers;
+//   - segments of up to kSegTiny elements are sorted by one thread each in registers, and finished
+//     by comparing the suffixes directly where their keys agree;
 //   - segments of up to kSegSmall elements are sorted entirely in shared memory: a block takes the
 //     segments that start in one kSegChunk-wide range of list positions (at most kSegCap elements)
 //     and radix-sorts them by (segment, subkey) with 8-bit digits, the keys travelling in registers
@@ -17,6 +18,7 @@
 
 #include <utility>
 
+#include "alphabet.cuh"
 #include "primitives.cuh"
 
 namespace sadcs {
@@ -167,12 +169,42 @@ __global__ void __launch_bounds__(256) segDigitBase(uint32_t* __restrict__ hist,
     row[threadIdx.x] = begin[blockIdx.x % segments] + inclusive - v;
 }
 
+// Suffixes i and j of one text compared from their characters at `from` on, up to kDirectWords stream
+// words: -1 or 1, or 0 if they agree so far.
+#ifndef SADCS_DIRECT_WORDS
+#define SADCS_DIRECT_WORDS 8
+#endif
+constexpr uint32_t kDirectList = 8u << 20;
+__device__ __noinline__ int directOrder(const TextSet& texts, uint32_t i, uint32_t j, uint32_t from) {
+    const uint32_t b = texts.bits, perWord = 64 / b;
+    const uint32_t end = texts.endOf(i), shorter = end - max(i, j);  // characters of the shorter suffix
+    uint64_t at = from;
+    for (int w = 0; w < SADCS_DIRECT_WORDS; w++, at += perWord) {
+        if (at >= shorter) return i > j ? -1 : 1;  // one ends: the shorter is the smaller
+        const uint32_t bits = static_cast<uint32_t>(min(shorter - at, static_cast<uint64_t>(perWord))) * b;
+        const uint64_t diff = (streamBits(texts.packed, (i + at) * b) ^ streamBits(texts.packed, (j + at) * b)) >> (64 - bits);
+        if (diff) {
+            // the highest differing bit belongs to the smaller suffix's 0
+            const uint64_t x = streamBits(texts.packed, (i + at) * b) >> (64 - bits);
+            return (x >> (63 - __clzll(static_cast<long long>(diff)))) & 1 ? 1 : -1;
+        }
+    }
+    return 0;
+}
+
 // Segments of 2 to kSegTiny elements, one thread each: keys and values into registers, sorted
-// by compare-exchange at fixed register indices (an insertion sort unrolled for kSegTiny), written
-// back in place. On genome-like text most groups left after the first pass are a repeat and its
-// copies (2-4 members), which the block-wide radix sort would take 4 to 8 passes over.
-__global__ void __launch_bounds__(256) segSortTiny(const uint32_t* __restrict__ heads, uint32_t segments,
-                                                   uint64_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+// by compare-exchange at fixed register indices (an insertion sort unrolled for kSegTiny). With kDirect,
+// elements whose keys agree (they share their first `depth` characters) are then compared directly, up to
+// kDirectWords words of the code stream further, instead of staying listed for more passes: on
+// genome-like text most groups left after the first pass are a repeat and its copies (2-4 members),
+// which agree for about a hundred characters. A sorted segment's keys are replaced by
+// numbers that differ where the order is known, so members that still agree stay a group, which
+// shares `depth` characters as every group of the pass does. tied counts the elements compared directly.
+// Written back in place.
+template <bool kDirect>
+__global__ void __launch_bounds__(256) segSortTiny(const uint32_t* __restrict__ heads, uint32_t segments, TextSet texts,
+                                                   uint32_t depth, uint64_t* __restrict__ keys,
+                                                   uint32_t* __restrict__ vals, uint32_t* __restrict__ tied) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= segments) return;
     const uint32_t begin = heads[k], size = heads[k + 1] - begin;
@@ -199,6 +231,42 @@ __global__ void __launch_bounds__(256) segSortTiny(const uint32_t* __restrict__ 
                     val[j - 1] = val[j];
                     val[j] = tv;
                 }
+            }
+        }
+    }
+    if constexpr (kDirect) {
+        uint32_t equal = 0;  // bit i: elements i and i + 1 have the same key
+#pragma unroll
+        for (uint32_t i = 0; i + 1 < kSegTiny; i++) {
+            if (i + 1 < size && key[i] == key[i + 1]) equal |= 1u << i;
+        }
+        if (equal) {
+            atomicAdd(tied, static_cast<uint32_t>(__popc(equal | (equal << 1))));
+            uint32_t same = equal;  // bit i: elements i and i + 1 are not known to differ
+            for (uint32_t round = 1; round < size; round++) {  // exchanges of neighbours until none is left
+                bool exchanged = false;
+                same = equal;
+#pragma unroll
+                for (uint32_t i = 0; i + 1 < kSegTiny; i++) {
+                    if ((equal >> i) & 1) {
+                        const int order = directOrder(texts, samplePosition(val[i]), samplePosition(val[i + 1]), depth);
+                        if (order) same &= ~(1u << i);
+                        if (order > 0) {
+                            const uint32_t tv = val[i];
+                            val[i] = val[i + 1];
+                            val[i + 1] = tv;
+                            exchanged = true;
+                        }
+                    }
+                }
+                if (!exchanged || size == 2) break;
+                same = equal;  // known only after a round without an exchange
+            }
+            uint64_t number = 0;
+#pragma unroll
+            for (uint32_t i = 0; i < kSegTiny; i++) {
+                if (i > 0 && !((same >> (i - 1)) & 1)) number++;
+                key[i] = number;
             }
         }
     }
@@ -413,16 +481,18 @@ struct SegBuffers {
     uint32_t* perSeg;   // 2 * u words (free key buffer): big flags and tile counts per segment
     uint32_t* scratch;  // scratchWords words, at least segScratchWords(u)
     size_t scratchWords;
-    uint32_t* counter;  // device words [0..3]
+    uint32_t* counter;  // device words [0..3]; [3]: elements that segSortTiny compared directly
     uint32_t* scanScratch;
+    bool* compared;     // (host) set when segSortTiny<true> ran: counter[3] holds its count
 };
 
-// Sorts the list (keys, vals: u elements in segments of equal grp) by key inside each segment.
+// Sorts the list (keys, vals: u elements, compact sample indices, in segments of equal grp) by key inside
+// each segment; elements of one segment with equal keys share their first `depth` characters.
 // Big segments use the alternates as the other buffer of their passes; the result is left in
 // keys/vals (pointers unchanged). hostWords: page-locked words for counts.
 inline cudaError_t segmentedSort(const uint32_t* grp, uint32_t u, uint64_t* keys, uint32_t* vals, uint64_t* keysAlt,
-                                 uint32_t* valsAlt, int keyBits, SegBuffers b, uint32_t* hostWords,
-                                 cudaStream_t stream) {
+                                 uint32_t* valsAlt, int keyBits, const TextSet& texts, uint32_t depth, SegBuffers b,
+                                 uint32_t* hostWords, cudaStream_t stream) {
     if (u <= 1) return cudaSuccess;
     SADCS_TRY(launch(segMarkHeads, ceilDiv(u, 256), 256, 0, stream, grp, u, b.flags));
     SADCS_TRY((deviceScan<OpSum, false>(b.flags, b.flags, u, b.scanScratch, b.counter, stream)));
@@ -445,7 +515,21 @@ inline cudaError_t segmentedSort(const uint32_t* grp, uint32_t u, uint64_t* keys
         return cudaFuncSetAttribute(segSortSmall, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(segSortSharedBytes()));
     }));
-    SADCS_TRY(launch(segSortTiny, ceilDiv(segments, 256), 256, 0, stream, b.heads, segments, keys, vals));
+    // Direct comparisons pay where the list is long (a pass over it costs DRAM traffic) and mostly pairs and
+    // triples: 2 GiB of genome-like text (59M samples listed, groups of 2.2) ranks in 49.8 ms against
+    // 58.2, five doubling rounds fewer; elsewhere they are made again in every pass for groups that
+    // stay (48 MiB of versions of one document, groups of 48: 15.9 ms against 13.5) or come on top of the
+    // passes that larger groups need anyway (256 MiB of natural-language-like text: 17.3 against 16.9).
+    const bool direct = u >= kDirectList && u <= 3 * static_cast<uint64_t>(segments);
+    if (direct) {
+        *b.compared = true;
+        SADCS_TRY(cudaMemsetAsync(b.counter + 3, 0, sizeof(uint32_t), stream));
+        SADCS_TRY(launch(segSortTiny<true>, ceilDiv(segments, 256), 256, 0, stream, b.heads, segments, texts, depth, keys,
+                         vals, b.counter + 3));
+    } else {
+        SADCS_TRY(launch(segSortTiny<false>, ceilDiv(segments, 256), 256, 0, stream, b.heads, segments, texts, depth, keys,
+                         vals, b.counter + 3));
+    }
     SADCS_TRY(launch(segSortSmall, ceilDiv(u, kSegChunk), kSegThreads, segSortSharedBytes(), stream, b.heads,
                      segments, keys, vals, keys, vals, keyBits));
     if (big == 0) return cudaSuccess;
