@@ -311,7 +311,8 @@ __global__ void __launch_bounds__(256) rankRefineScan(uint32_t* __restrict__ agg
     if (threadIdx.x == 0) *total = carryKept;
 }
 
-// Each tile again with its carries: ids into the rank array, kept elements compacted into out.
+// Each tile again with its carries: ids into the rank array, kept elements compacted into out. A list of
+// one tile has no carries (agg null) and leaves its kept count in total.
 __global__ void __launch_bounds__(kRefineThreads) rankRefineApply(const uint32_t* __restrict__ grp,
                                                                   const uint64_t* __restrict__ key,
                                                                   const uint32_t* __restrict__ lst, uint32_t u,
@@ -320,7 +321,8 @@ __global__ void __launch_bounds__(kRefineThreads) rankRefineApply(const uint32_t
                                                                   uint32_t* __restrict__ ranks,
                                                                   uint32_t* __restrict__ out,
                                                                   uint32_t* __restrict__ grpOut, uint32_t writeAll,
-                                                                  uint64_t* __restrict__ pairs) {
+                                                                  uint64_t* __restrict__ pairs,
+                                                                  uint32_t* __restrict__ total) {
     __shared__ uint32_t warpTotals[32];
     __shared__ uint32_t incOld[kRefineThreads], incNew[kRefineThreads];
     const uint32_t base = blockIdx.x * kRefineTile + threadIdx.x * kRefineItems;
@@ -337,9 +339,10 @@ __global__ void __launch_bounds__(kRefineThreads) rankRefineApply(const uint32_t
     incOld[threadIdx.x] = io;
     incNew[threadIdx.x] = iw;
     __syncthreads();
-    uint32_t runOld = max(agg[blockIdx.x], threadIdx.x ? incOld[threadIdx.x - 1] : 0u);
-    uint32_t runNew = max(agg[tiles + blockIdx.x], threadIdx.x ? incNew[threadIdx.x - 1] : 0u);
-    uint32_t at = agg[2 * tiles + blockIdx.x] + ic - kept;
+    uint32_t runOld = max(agg ? agg[blockIdx.x] : 0u, threadIdx.x ? incOld[threadIdx.x - 1] : 0u);
+    uint32_t runNew = max(agg ? agg[tiles + blockIdx.x] : 0u, threadIdx.x ? incNew[threadIdx.x - 1] : 0u);
+    uint32_t at = (agg ? agg[2 * tiles + blockIdx.x] : 0u) + ic - kept;
+    if (!agg && threadIdx.x == 0) *total = totalKept;
     uint32_t items[kRefineItems];
     if (base + kRefineItems <= u) {
 #pragma unroll
@@ -533,12 +536,15 @@ inline cudaError_t rankSample(const uint8_t* text, const TextSet& texts, uint32_
         // The next pass reads ranks of other samples when it is a doubling round.
         const bool writeAll = doubling || depth + passTexts.keyChars >= kV;
         const uint32_t refineTiles = ceilDiv(u, kRefineTile);
-        SADCS_TRY(launch(rankRefineReduce, refineTiles, kRefineThreads, 0, stream, b.grp, key, u, refineTiles, b.aux1));
-        SADCS_TRY(launch(rankRefineScan, 1, 256, 0, stream, b.aux1, refineTiles, b.counter));
+        if (refineTiles > 1) {
+            SADCS_TRY(launch(rankRefineReduce, refineTiles, kRefineThreads, 0, stream, b.grp, key, u, refineTiles, b.aux1));
+            SADCS_TRY(launch(rankRefineScan, 1, 256, 0, stream, b.aux1, refineTiles, b.counter));
+        }
         // A large pass writes its ranks through pairs in the free key buffer (bucketed, below).
         const bool bucketed = u >= kBucketedRankWrites && slots >= kBucketedRankSlots && slots <= b.keyEntries;
         SADCS_TRY(launch(rankRefineApply, refineTiles, kRefineThreads, 0, stream, b.grp, key, lst, u, slots, refineTiles,
-                         b.aux1, ranks, lstAlt, b.aux2, writeAll ? 1u : 0u, bucketed ? keyAlt : nullptr));
+                         refineTiles > 1 ? b.aux1 : nullptr, ranks, lstAlt, b.aux2, writeAll ? 1u : 0u,
+                         bucketed ? keyAlt : nullptr, b.counter));
         if (bucketed) {
             // the sorted keys are dead now: they become the slice-major pair array
             const uint32_t shift = sliceShift(slots);

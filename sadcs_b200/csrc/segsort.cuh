@@ -75,6 +75,53 @@ __global__ void segCollectHeads(const uint32_t* __restrict__ grp, const uint32_t
     if (i == 0) heads[segments] = u;
 }
 
+// The heads of a list of at most kSegOneBlock elements, in one block: heads[0 .. S] as segCollectHeads
+// leaves them, counter[0..2] = S, the big segments and their tiles. A short list's pass is bound by its
+// launches and the waits for its counts: one launch and one wait here, against nine and two.
+constexpr uint32_t kSegOneBlock = 16384;
+constexpr int kSegOneThreads = 1024;
+__global__ void __launch_bounds__(kSegOneThreads) segHeadsOneBlock(const uint32_t* __restrict__ grp, uint32_t u,
+                                                                   uint32_t* __restrict__ heads,
+                                                                   uint32_t* __restrict__ counter) {
+    __shared__ uint32_t warpTotals[32];
+    __shared__ uint32_t sBig, sTiles;
+    constexpr uint32_t kItems = kSegOneBlock / kSegOneThreads;
+    if (threadIdx.x == 0) sBig = sTiles = 0;
+    const uint32_t base = threadIdx.x * kItems;
+    uint32_t starts = 0;  // bit k: a segment starts at base + k
+    uint32_t before = base > 0 && base <= u ? grp[base - 1] : 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kItems; k++) {
+        const uint32_t i = base + k;
+        if (i < u) {
+            const uint32_t g = grp[i];
+            if (i == 0 || g != before) starts |= 1u << k;
+            before = g;
+        }
+    }
+    uint32_t segments;
+    uint32_t at = blockInclusiveScan<OpSum>(__popc(starts), warpTotals, segments) - __popc(starts);
+#pragma unroll
+    for (uint32_t k = 0; k < kItems; k++) {
+        if ((starts >> k) & 1) heads[at++] = base + k;
+    }
+    if (threadIdx.x == 0) heads[segments] = u;
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < segments; k += kSegOneThreads) {
+        const uint32_t size = heads[k + 1] - heads[k];
+        if (size > kSegSmall) {
+            atomicAdd(&sBig, 1u);
+            atomicAdd(&sTiles, (size + kSortTile - 1) / kSortTile);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        counter[0] = segments;
+        counter[1] = sBig;
+        counter[2] = sTiles;
+    }
+}
+
 // Per segment k: bigFlag[k] = size > kSegSmall, tiles[k] = its tiles if big (both scanned later).
 __global__ void segClassify(const uint32_t* __restrict__ heads, uint32_t segments, uint32_t* __restrict__ bigFlag,
                             uint32_t* __restrict__ tiles) {
@@ -494,19 +541,32 @@ inline cudaError_t segmentedSort(const uint32_t* grp, uint32_t u, uint64_t* keys
                                  uint32_t* valsAlt, int keyBits, const TextSet& texts, uint32_t depth, SegBuffers b,
                                  uint32_t* hostWords, cudaStream_t stream) {
     if (u <= 1) return cudaSuccess;
-    SADCS_TRY(launch(segMarkHeads, ceilDiv(u, 256), 256, 0, stream, grp, u, b.flags));
-    SADCS_TRY((deviceScan<OpSum, false>(b.flags, b.flags, u, b.scanScratch, b.counter, stream)));
-    SADCS_TRY(cudaMemcpyAsync(hostWords, b.counter, 4, cudaMemcpyDeviceToHost, stream));
-    SADCS_TRY(cudaStreamSynchronize(stream));
+    // A list of up to kSegOneBlock elements: one launch and one wait (the ranking of a 64 KiB text, with the
+    // one-tile refinement, 0.67 -> 0.54 ms); its big segments' tables are made only if it has some.
+    const bool oneBlock = u <= kSegOneBlock;
+    if (oneBlock) {
+        SADCS_TRY(launch(segHeadsOneBlock, 1, kSegOneThreads, 0, stream, grp, u, b.heads, b.counter));
+        SADCS_TRY(cudaMemcpyAsync(hostWords, b.counter, 12, cudaMemcpyDeviceToHost, stream));
+        SADCS_TRY(cudaStreamSynchronize(stream));
+    } else {
+        SADCS_TRY(launch(segMarkHeads, ceilDiv(u, 256), 256, 0, stream, grp, u, b.flags));
+        SADCS_TRY((deviceScan<OpSum, false>(b.flags, b.flags, u, b.scanScratch, b.counter, stream)));
+        SADCS_TRY(cudaMemcpyAsync(hostWords, b.counter, 4, cudaMemcpyDeviceToHost, stream));
+        SADCS_TRY(cudaStreamSynchronize(stream));
+        SADCS_TRY(launch(segCollectHeads, ceilDiv(u, 256), 256, 0, stream, grp, b.flags, u, hostWords[0], b.heads));
+    }
     const uint32_t segments = hostWords[0];
-    SADCS_TRY(launch(segCollectHeads, ceilDiv(u, 256), 256, 0, stream, grp, b.flags, u, segments, b.heads));
     uint32_t* bigFlag = b.perSeg;
     uint32_t* tiles = b.perSeg + u;
-    SADCS_TRY(launch(segClassify, ceilDiv(segments, 256), 256, 0, stream, b.heads, segments, bigFlag, tiles));
-    SADCS_TRY((deviceScan<OpSum, false>(bigFlag, bigFlag, segments, b.scanScratch, b.counter + 1, stream)));
-    SADCS_TRY((deviceScan<OpSum, false>(tiles, tiles, segments, b.scanScratch, b.counter + 2, stream)));
-    SADCS_TRY(cudaMemcpyAsync(hostWords + 1, b.counter + 1, 8, cudaMemcpyDeviceToHost, stream));
-    SADCS_TRY(cudaStreamSynchronize(stream));
+    if (!oneBlock || hostWords[1]) {
+        SADCS_TRY(launch(segClassify, ceilDiv(segments, 256), 256, 0, stream, b.heads, segments, bigFlag, tiles));
+        SADCS_TRY((deviceScan<OpSum, false>(bigFlag, bigFlag, segments, b.scanScratch, b.counter + 1, stream)));
+        SADCS_TRY((deviceScan<OpSum, false>(tiles, tiles, segments, b.scanScratch, b.counter + 2, stream)));
+    }
+    if (!oneBlock) {
+        SADCS_TRY(cudaMemcpyAsync(hostWords + 1, b.counter + 1, 8, cudaMemcpyDeviceToHost, stream));
+        SADCS_TRY(cudaStreamSynchronize(stream));
+    }
     const uint32_t big = hostWords[1], bigTiles = hostWords[2];
 
     // Small segments, in place.
