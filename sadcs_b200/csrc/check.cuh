@@ -60,7 +60,8 @@ __global__ void checkOrder(const uint8_t* __restrict__ text, const uint32_t* __r
 //
 // The same conditions, for the common case that they hold: no failing index is kept, so the inverse
 // suffix array needs no order among equal entries and is written slice by slice (scatterBySlices), and
-// one pass reads each entry's inverse once for both conditions. A suffix array that fails goes to the
+// two passes check the conditions: the first characters in text order, then the permutation
+// and the order of neighbours from one read of each entry's inverse. A suffix array that fails goes to the
 // kernels above, which find the first failing index. isa starts as all ones, which no entry is.
 struct InversePairs {
     const uint32_t* __restrict__ sa;
@@ -71,40 +72,63 @@ struct InversePairs {
     }
 };
 
-// failed != 0 unless every i has sa[i] < n, isa[sa[i]] = i (so sa is a permutation: n distinct slots are
-// owned), and neighbours in order by (first character, inverse of the suffix after it). Bound by its two
-// random reads per entry, isa[sa[i]] (with the entry after it, usually the same sector) and the
-// character: each is read once and handed to the entry before by the warp, the last lane's by
-// memory.
+// failed != 0 unless the suffix at every inverse rank starts with the character of that rank: rank i
+// belongs to the byte c whose range [starts[c], starts[c + 1]) of the text's sorted bytes holds it. In
+// text order, so nothing is read at random.
 constexpr int kVerifyThreads = 256;
-__global__ void __launch_bounds__(kVerifyThreads) checkVerify(const uint8_t* __restrict__ text,
-                                                              const uint32_t* __restrict__ sa, uint32_t n,
+__global__ void __launch_bounds__(kVerifyThreads) checkFirst(const uint8_t* __restrict__ text, uint32_t n,
+                                                             const uint32_t* __restrict__ isa,
+                                                             const uint32_t* __restrict__ starts,
+                                                             uint32_t* __restrict__ failed) {
+    __shared__ uint32_t first[257];
+    first[threadIdx.x] = starts[threadIdx.x];
+    if (threadIdx.x == 0) first[256] = n;
+    __syncthreads();
+    bool ok = true;
+    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kVerifyThreads;
+    for (uint64_t p = static_cast<uint64_t>(blockIdx.x) * kVerifyThreads + threadIdx.x; p < n; p += stride) {
+        const uint32_t r = __ldcs(isa + p), c = text[p];
+        ok = ok && r >= first[c] && r < first[c + 1];
+    }
+    if (!ok) *failed = 1;
+}
+
+// failed != 0 unless every i has sa[i] < n, isa[sa[i]] = i (so sa is a permutation: n distinct slots are
+// owned), and neighbours of the same first character (by starts; checkFirst says that they have it) in
+// order by the inverse of the suffix after it. Bound by its one random read per entry, isa[sa[i]] with
+// the entry after it (usually the same sector): read once and handed to the entry before by the warp,
+// the last lane's by memory. The characters read here too made it 4.5 ms at 128 MiB.
+__global__ void __launch_bounds__(kVerifyThreads) checkVerify(const uint32_t* __restrict__ sa, uint32_t n,
                                                               const uint32_t* __restrict__ isa,
+                                                              const uint32_t* __restrict__ starts,
                                                               uint32_t* __restrict__ failed) {
-    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kVerifyThreads + threadIdx.x;
+    __shared__ uint32_t boundary[kVerifyThreads / 32];  // bit: a byte's range starts at the place after this one
+    const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kVerifyThreads, i = base + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31;
-    // (first character, 1 + inverse of the suffix after it, 0 for the empty one) of entry e; owned: isa says so too
-    const auto look = [&](uint64_t e, uint32_t& c, uint32_t& after, bool& owned) {
+    if (threadIdx.x < kVerifyThreads / 32) boundary[threadIdx.x] = 0;
+    __syncthreads();
+    static_assert(kVerifyThreads == 256, "one thread per byte value");
+    const uint64_t at = starts[threadIdx.x];
+    if (at > base && at <= base + kVerifyThreads) {
+        const uint32_t k = static_cast<uint32_t>(at - 1 - base);
+        atomicOr(&boundary[k >> 5], 1u << (k & 31));
+    }
+    // 1 + the inverse of the suffix after entry e's first character, 0 for the empty one
+    const auto look = [&](uint64_t e, uint32_t& after) {
         const uint32_t p = sa[e];
-        c = after = 0;
-        owned = p < n;
-        if (owned) {
-            owned = isa[p] == e;
-            c = text[p];
-            after = p + 1 < n ? isa[p + 1] + 1 : 0;
-        }
+        after = 0;
+        if (p >= n) return false;
+        after = p + 1 < n ? isa[p + 1] + 1 : 0;
+        return isa[p] == e;
     };
-    uint32_t c = 0, after = 0;
-    bool owned = true;
-    if (i < n) look(i, c, after, owned);
-    uint32_t c2 = __shfl_down_sync(0xffffffffu, c, 1), after2 = __shfl_down_sync(0xffffffffu, after, 1);
-    bool ok = owned;
+    uint32_t after = 0;
+    bool ok = true;
+    if (i < n) ok = look(i, after);
+    uint32_t after2 = __shfl_down_sync(0xffffffffu, after, 1);
+    __syncthreads();
     if (i + 1 < n) {
-        if (lane == 31) {
-            bool owned2;
-            look(i + 1, c2, after2, owned2);
-        }
-        ok = ok && (c < c2 || (c == c2 && after < after2));
+        if (lane == 31) look(i + 1, after2);
+        ok = ok && (after < after2 || ((boundary[threadIdx.x >> 5] >> lane) & 1));
     }
     if (!ok) *failed = 1;
 }

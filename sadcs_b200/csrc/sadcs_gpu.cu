@@ -1173,7 +1173,7 @@ int sadcs_gpu_check_suffix_array(const uint8_t* d_text, int64_t n, const uint32_
     unsigned long long host[3] = {kNoFailure, kNoFailure, kNoFailure};
     cudaError_t error;
     if ((error = workspace(&isa, 4 * static_cast<size_t>(n), st)) != cudaSuccess) return failed("allocating check buffers", error);
-    if ((error = workspace(&words, 4 * sizeof(unsigned long long), st)) != cudaSuccess) {
+    if ((error = workspace(&words, 4 * sizeof(unsigned long long) + 256 * sizeof(uint32_t), st)) != cudaSuccess) {
         cudaFreeAsync(isa, st);
         return failed("allocating check buffers", error);
     }
@@ -1184,8 +1184,9 @@ int sadcs_gpu_check_suffix_array(const uint8_t* d_text, int64_t n, const uint32_
     }
     const uint32_t blocks = (count + 255) / 256;
     uint32_t* failedWord = reinterpret_cast<uint32_t*>(words + 3);
+    uint32_t* starts = reinterpret_cast<uint32_t*>(words + 4);  // of every byte in the sorted text
     uint32_t hostFailed = 0;
-    error = cudaMemsetAsync(failedWord, 0, sizeof(uint32_t), st);
+    error = cudaMemsetAsync(failedWord, 0, 2 * sizeof(uint32_t) + 256 * sizeof(uint32_t), st);
     if (error == cudaSuccess) error = cudaMemsetAsync(words, 0xFF, 3 * sizeof(unsigned long long), st);
     if (error == cudaSuccess) error = cudaMemsetAsync(isa, pairs ? 0xFF : 0, 4 * static_cast<size_t>(count), st);
     if (error == cudaSuccess) {
@@ -1193,7 +1194,11 @@ int sadcs_gpu_check_suffix_array(const uint8_t* d_text, int64_t n, const uint32_
                                         reinterpret_cast<uint32_t*>(pairs + count), st)
                       : launch(checkScatter, blocks, 256, 0, st, d_sa, count, isa, words);
     }
-    if (error == cudaSuccess) error = launch(checkVerify, ceilDiv(count, kVerifyThreads), kVerifyThreads, 0, st, d_text, d_sa, count, isa, failedWord);
+    const uint32_t stridedBlocks = std::min<uint32_t>(ceilDiv(count, 256 * 16), 148 * 8);
+    if (error == cudaSuccess) error = launch(byteHistogram, stridedBlocks, 256, 0, st, d_text, count, starts);
+    if (error == cudaSuccess) error = launch(inverseChunkBases, 1, 256, 0, st, starts, 1u);
+    if (error == cudaSuccess) error = launch(checkFirst, stridedBlocks, kVerifyThreads, 0, st, d_text, count, isa, starts, failedWord);
+    if (error == cudaSuccess) error = launch(checkVerify, ceilDiv(count, kVerifyThreads), kVerifyThreads, 0, st, d_sa, count, isa, starts, failedWord);
     if (error == cudaSuccess) error = cudaMemcpyAsync(&hostFailed, failedWord, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
     if (error == cudaSuccess) error = cudaStreamSynchronize(st);
     const char* why = nullptr;
