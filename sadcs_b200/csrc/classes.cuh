@@ -118,12 +118,14 @@ __device__ __forceinline__ uint64_t carriedWord(const uint64_t* __restrict__ pac
 // and each slice's writes stay within the list's L2-sized slice.
 constexpr uint32_t kSampleSliceShift = 23;  // 8M ranks = 32 MB of the list per slice
 #ifndef SADCS_CARRY_SLICE_SHIFT
-#define SADCS_CARRY_SLICE_SHIFT 22  // with carried words: 4M ranks = 16 + 32 MB per slice (tuning)
+// With carried words: 1M ranks = 4 + 8 MB per slice, more where that gives more than kMaxSlices slices
+// (2 GiB: 2M, class phase 46.5 ms; 47.5 with 4M) (tuning).
+#define SADCS_CARRY_SLICE_SHIFT 20
 #endif
 constexpr uint32_t kCarrySampleSliceShift = SADCS_CARRY_SLICE_SHIFT;
 constexpr uint32_t kMaxSampleSlices = kMaxSlices;
 
-// The slice width (as a shift) for `live` samples: at least 8M ranks (4M with carried words), at
+// The slice width (as a shift) for `live` samples: at least 8M ranks (1M with carried words), at
 // most kMaxSampleSlices slices.
 inline uint32_t sampleSliceShift(uint64_t live, bool carry) {
     uint32_t shift = carry ? kCarrySampleSliceShift : kSampleSliceShift;

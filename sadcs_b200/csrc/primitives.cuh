@@ -304,10 +304,12 @@ __global__ void __launch_bounds__(kPairThreads) sliceScatter(const uint64_t* __r
     }
 }
 
-// The slice width (as a shift) for a target of `entries` words: 4M words = 16 MB (at 3 GiB 0.6 ms
-// less ranking than 8M), more where that would give more than kMaxSlices slices.
+// The slice width (as a shift) for a target of `entries` words: 1M words = 4 MB, more where that would
+// give more than kMaxSlices slices (2 GiB of genome-like text, 470M samples, then 2M: its ranking takes
+// 49.06 ms, with 4M 49.38; 100 MB of protein-like text 2.65 and 2.70; at 3 GiB 4M took 0.6 ms less than
+// 8M).
 #ifndef SADCS_SLICE_SHIFT
-#define SADCS_SLICE_SHIFT 22
+#define SADCS_SLICE_SHIFT 20
 #endif
 inline uint32_t sliceShift(uint64_t entries) {
     uint32_t shift = SADCS_SLICE_SHIFT;
@@ -330,7 +332,7 @@ cudaError_t scatterBySlices(const Source& source, uint32_t n, uint32_t* out, uin
 }
 
 #ifndef SADCS_VOTE_SHARE
-#define SADCS_VOTE_SHARE 64
+#define SADCS_VOTE_SHARE 80
 #endif
 
 // ---- radix pass (onesweep) ------------------------------------------------------------------
@@ -406,16 +408,21 @@ struct ManySegments {
 // same elements only, so that values are not held in registers through ranking and look-back).
 // Storers write keys (when kKeys) and values at output positions.
 // Tiles resident per SM the register budget is set for: a loader may ask for its own number
-// (kTilesPerSm), otherwise SADCS_SORT_TILES (tuning).
+// (kTilesPerSm), otherwise 4 (64 registers) for the sorts of many segments, which are long (1.0 ms off
+// the 4096-text batch's ranking of 75.4 against 3), and 3 (80 registers) for those of one, whose few
+// tiles on a small text run one by one (8 MiB of uniform bytes: ranking 0.43 ms, 0.49 with 4).
 #ifndef SADCS_SORT_TILES
 #define SADCS_SORT_TILES 3
 #endif
-template <class Loader, class = void>
+#ifndef SADCS_SEGMENT_SORT_TILES
+#define SADCS_SEGMENT_SORT_TILES 4
+#endif
+template <class Loader, class Segments, class = void>
 struct SortTilesPerSm {
-    static constexpr int value = SADCS_SORT_TILES;
+    static constexpr int value = std::is_same<Segments, OneSegment>::value ? SADCS_SORT_TILES : SADCS_SEGMENT_SORT_TILES;
 };
-template <class Loader>
-struct SortTilesPerSm<Loader, std::void_t<decltype(Loader::kTilesPerSm)>> {
+template <class Loader, class Segments>
+struct SortTilesPerSm<Loader, Segments, std::void_t<decltype(Loader::kTilesPerSm)>> {
     static constexpr int value = Loader::kTilesPerSm;
 };
 
@@ -448,7 +455,8 @@ struct LoaderCarries<Loader, std::void_t<decltype(Loader::kCarry)>> {
 // mostly distinct and match where they repeat (kVoteShare). Ranking
 // with votes in every pass of the first sort: 100 MB of protein-like text 2.85 -> 2.66 ms, 2 GiB of
 // genome-like text 61.2 -> 58.7, 8 MiB of uniform bytes 0.45 -> 0.41, but 256 MiB of
-// natural-language-like text 16.9 -> 17.3; by the rule 2.69, 58.3, 0.42 and 16.6. The class passes' few
+// natural-language-like text 16.9 -> 17.3; by the rule 2.69, 58.3, 0.42 and 16.5
+// (a share of 128 sends the protein-like text's digits to the match: 2.99). The class passes' few
 // digits match (2 GiB of genome-like text: 49.1 ms, 53.4 with votes).
 constexpr uint32_t kVoteShare = SADCS_VOTE_SHARE;  // votes where two random keys share a digit in fewer than 1 of kVoteShare cases
 __device__ __forceinline__ uint32_t digitPeers(uint32_t digit, bool valid) {
@@ -473,7 +481,7 @@ struct LoaderVotes<Loader, std::void_t<decltype(std::declval<const Loader&>().vo
 };
 
 template <class Key, class Loader, class Storer, class Segments = OneSegment>
-__global__ void __launch_bounds__(kSortThreads, SortTilesPerSm<Loader>::value) radixOnesweep(Loader ld, Storer st, Segments segs,
+__global__ void __launch_bounds__(kSortThreads, SortTilesPerSm<Loader, Segments>::value) radixOnesweep(Loader ld, Storer st, Segments segs,
                                                                  const uint32_t* __restrict__ digitBase,
                                                                  uint32_t* __restrict__ status,
                                                                  uint32_t* __restrict__ tileCounter,

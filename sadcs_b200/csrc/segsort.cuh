@@ -24,7 +24,7 @@
 namespace sadcs {
 
 #ifndef SADCS_SEGSORT_BLOCKS
-#define SADCS_SEGSORT_BLOCKS 4  // resident blocks per SM the register budget is set for (tuning)
+#define SADCS_SEGSORT_BLOCKS 5  // resident blocks per SM the register budget is set for (tuning)
 #endif
 
 #ifndef SADCS_SEGSORT_SMALL
