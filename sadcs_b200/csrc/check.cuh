@@ -167,7 +167,7 @@ constexpr uint32_t kCoarse = 2048;           // entries of the walk's table of f
 constexpr uint32_t kNoPiece = 0xFFFFFFFFu;
 
 // The splitter row of rows [128q, 128q + 128).
-__device__ __forceinline__ uint32_t splitterRow(uint32_t q) {
+__host__ __device__ __forceinline__ uint32_t splitterRow(uint32_t q) {
     uint32_t h = q * 0x9E3779B1u;
     h ^= h >> 15;
     h *= 0x85EBCA77u;
@@ -261,12 +261,29 @@ __global__ void __launch_bounds__(kWalkThreads) inverseWalk(const uint32_t* __re
     }
 }
 
+// One round of pointer jumping for one piece: where the piece after it leads, the lengths added (mod 2^32).
+__host__ __device__ __forceinline__ uint64_t jumpOver(uint64_t mine, uint64_t next) {
+    return (next & 0xFFFFFFFF00000000ull) | static_cast<uint32_t>(static_cast<uint32_t>(mine) + static_cast<uint32_t>(next));
+}
+
 // One round of pointer jumping over the pieces and the end.
 __global__ void inverseJump(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, uint32_t pieces) {
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q > pieces + 1) return;
-    const uint64_t mine = in[q], next = in[mine >> 32];
-    out[q] = (next & 0xFFFFFFFF00000000ull) | static_cast<uint32_t>(static_cast<uint32_t>(mine) + static_cast<uint32_t>(next));
+    const uint64_t mine = in[q];
+    out[q] = jumpOver(mine, in[mine >> 32]);
+}
+
+// The first place in the text of a chunk of `length` characters that follow `before` characters of its
+// piece; false if it has none. toEnd: the piece's entry after the jumps. Only a BWT that does not
+// invert has pieces that never reach the end (they lie on cycles of psi, and the lengths added up over their
+// laps mean nothing); the characters of those that do reach it are on one way, so their sum is exact.
+__host__ __device__ __forceinline__ bool chunkPlace(uint64_t toEnd, uint32_t pieces, uint32_t n, uint32_t before,
+                                                    uint32_t length, uint64_t& at) {
+    const uint32_t left = static_cast<uint32_t>(toEnd);  // characters from the piece's start to the end
+    if (toEnd >> 32 != pieces + 1 || left > n || before > left || length > left - before) return false;
+    at = n - left + before;
+    return true;
 }
 
 // Every chunk to its place: the characters from its piece to the end of the text are known now. control[1]
@@ -274,16 +291,16 @@ __global__ void inverseJump(const uint64_t* __restrict__ in, uint64_t* __restric
 // the text are written as words.
 __global__ void __launch_bounds__(256) inverseSpell(const uint4* __restrict__ chunks, const uint2* __restrict__ owner,
                                                     const uint32_t* __restrict__ control, uint32_t maxChunks,
-                                                    const uint64_t* __restrict__ toEnd, uint32_t n,
-                                                    uint8_t* __restrict__ text) {
+                                                    const uint64_t* __restrict__ toEnd, uint32_t pieces,
+                                                    uint32_t n, uint8_t* __restrict__ text) {
     const uint32_t count = min(control[1], maxChunks);
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const uint2 o = owner[k];
     if (o.x == kNoPiece) return;
     const uint32_t length = (o.y - 1) % kChunkChars + 1, before = o.y - length;
-    const uint64_t at = static_cast<uint64_t>(n) - static_cast<uint32_t>(toEnd[o.x]) + before;
-    if (at + length > n) return;  // a piece that is not on the way from the primary row (a broken BWT)
+    uint64_t at;
+    if (!chunkPlace(toEnd[o.x], pieces, n, before, length, at)) return;
     const uint4 v = chunks[k];
     const uint32_t words[5] = {v.x, v.y, v.z, v.w, 0};
     uint8_t* to = text + at;
@@ -435,7 +452,7 @@ inline cudaError_t inverseBwt(const uint8_t* bwt, uint32_t n, uint32_t primary, 
                          jump[cur ^ 1], pieces));
     }
     SADCS_TRY(launch(inverseSpell, ceilDiv(inverseChunks(n), 256), 256, 0, stream, chunkData, owner, control, maxChunks,
-                     jump[cur], n, text));
+                     jump[cur], pieces, n, text));
     SADCS_TRY(cudaMemcpyAsync(hostWords, jump[cur] + pieces, 8, cudaMemcpyDeviceToHost, stream));
     SADCS_TRY(cudaMemcpyAsync(hostWords + 2, radix.control + 1, 4, cudaMemcpyDeviceToHost, stream));
     SADCS_TRY(cudaStreamSynchronize(stream));
