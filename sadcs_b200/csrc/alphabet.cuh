@@ -111,11 +111,15 @@ __global__ void __launch_bounds__(256) packCodes(const uint8_t* __restrict__ tex
 }
 
 // 64 bits of the code stream starting at stream bit `bit`.
-__device__ __forceinline__ uint64_t streamBits(const uint64_t* __restrict__ packed, uint64_t bit) {
+__host__ __device__ __forceinline__ uint64_t streamBits(const uint64_t* __restrict__ packed, uint64_t bit) {
     const uint64_t w = bit >> 6;
     const uint32_t o = static_cast<uint32_t>(bit & 63);
+#ifdef __CUDA_ARCH__
     const uint64_t hi = __ldg(packed + w);
     return o ? (hi << o) | (__ldg(packed + w + 1) >> (64 - o)) : hi;
+#else
+    return o ? (packed[w] << o) | (packed[w + 1] >> (64 - o)) : packed[w];
+#endif
 }
 
 // The code of character q: one word of the stream, two when the character straddles them.

@@ -216,33 +216,60 @@ __global__ void __launch_bounds__(256) segDigitBase(uint32_t* __restrict__ hist,
     row[threadIdx.x] = begin[blockIdx.x % segments] + inclusive - v;
 }
 
-// Suffixes i and j of one text compared from their characters at `from` on, up to kDirectWords stream
-// words: -1 or 1, or 0 if they agree so far.
+// Suffixes i and j of one text ending at `end`, compared from their characters at `from` on, up to
+// SADCS_DIRECT_WORDS stream words: -1 or 1, or 0 if they agree so far and neither has ended. One that ends
+// within the last word is decided too: left at 0 it would be equal to suffixes that differ from one another after its
+// end, and no order of the group would be consistent with that.
 #ifndef SADCS_DIRECT_WORDS
 #define SADCS_DIRECT_WORDS 8
 #endif
 constexpr uint32_t kDirectList = 8u << 20;
-__device__ __noinline__ int directOrder(const TextSet& texts, uint32_t i, uint32_t j, uint32_t from) {
-    const uint32_t b = texts.bits, perWord = 64 / b;
-    const uint32_t end = texts.endOf(i), shorter = end - max(i, j);  // characters of the shorter suffix
+__host__ __device__ __noinline__ int directOrder(const uint64_t* __restrict__ packed, uint32_t b, uint32_t end, uint32_t i,
+                                                 uint32_t j, uint32_t from) {
+    const uint32_t perWord = 64 / b, shorter = end - (i > j ? i : j);  // characters of the shorter suffix
     uint64_t at = from;
     for (int w = 0; w < SADCS_DIRECT_WORDS; w++, at += perWord) {
         if (at >= shorter) return i > j ? -1 : 1;  // one ends: the shorter is the smaller
-        const uint32_t bits = static_cast<uint32_t>(min(shorter - at, static_cast<uint64_t>(perWord))) * b;
-        const uint64_t diff = (streamBits(texts.packed, (i + at) * b) ^ streamBits(texts.packed, (j + at) * b)) >> (64 - bits);
-        if (diff) {
-            // the highest differing bit belongs to the smaller suffix's 0
-            const uint64_t x = streamBits(texts.packed, (i + at) * b) >> (64 - bits);
-            return (x >> (63 - __clzll(static_cast<long long>(diff)))) & 1 ? 1 : -1;
-        }
+        const uint32_t bits = (shorter - at < perWord ? static_cast<uint32_t>(shorter - at) : perWord) * b;
+        const uint64_t x = streamBits(packed, (i + at) * b) >> (64 - bits);
+        const uint64_t y = streamBits(packed, (j + at) * b) >> (64 - bits);
+        if (x != y) return x < y ? -1 : 1;
     }
-    return 0;
+    return at < shorter ? 0 : (i > j ? -1 : 1);
+}
+
+// The values of up to kSegTiny elements sorted by order (-1, 0 or 1) within the runs of equal keys, by
+// exchanges of neighbours. equal, bit i: elements i and i + 1 have the same key. Returns it without the
+// bits of neighbours that are now known to differ.
+template <class Order>
+__host__ __device__ __forceinline__ uint32_t orderEqual(uint32_t (&val)[kSegTiny], uint32_t size, uint32_t equal, Order order) {
+    uint32_t same = equal;
+    for (uint32_t round = 1; round < size; round++) {  // until a round exchanges nothing
+        bool exchanged = false;
+        same = equal;
+#pragma unroll
+        for (uint32_t i = 0; i + 1 < kSegTiny; i++) {
+            if ((equal >> i) & 1) {
+                const int o = order(val[i], val[i + 1]);
+                if (o) same &= ~(1u << i);
+                if (o > 0) {
+                    const uint32_t tv = val[i];
+                    val[i] = val[i + 1];
+                    val[i + 1] = tv;
+                    exchanged = true;
+                }
+            }
+        }
+        if (!exchanged || size == 2) break;
+        same = equal;  // known only after a round without an exchange
+    }
+    return same;
 }
 
 // Segments of 2 to kSegTiny elements, one thread each: keys and values into registers, sorted
 // by compare-exchange at fixed register indices (an insertion sort unrolled for kSegTiny). With kDirect,
 // elements whose keys agree (they share their first `depth` characters) are then compared directly, up to
-// kDirectWords words of the code stream further, instead of staying listed for more passes: on
+// SADCS_DIRECT_WORDS words of the code stream further, instead of staying listed for more passes: on
 // genome-like text most groups left after the first pass are a repeat and its copies (2-4 members),
 // which agree for about a hundred characters. A sorted segment's keys are replaced by
 // numbers that differ where the order is known, so members that still agree stay a group, which
@@ -289,26 +316,10 @@ __global__ void __launch_bounds__(256) segSortTiny(const uint32_t* __restrict__ 
         }
         if (equal) {
             atomicAdd(tied, static_cast<uint32_t>(__popc(equal | (equal << 1))));
-            uint32_t same = equal;  // bit i: elements i and i + 1 are not known to differ
-            for (uint32_t round = 1; round < size; round++) {  // exchanges of neighbours until none is left
-                bool exchanged = false;
-                same = equal;
-#pragma unroll
-                for (uint32_t i = 0; i + 1 < kSegTiny; i++) {
-                    if ((equal >> i) & 1) {
-                        const int order = directOrder(texts, samplePosition(val[i]), samplePosition(val[i + 1]), depth);
-                        if (order) same &= ~(1u << i);
-                        if (order > 0) {
-                            const uint32_t tv = val[i];
-                            val[i] = val[i + 1];
-                            val[i + 1] = tv;
-                            exchanged = true;
-                        }
-                    }
-                }
-                if (!exchanged || size == 2) break;
-                same = equal;  // known only after a round without an exchange
-            }
+            const uint32_t end = texts.endOf(samplePosition(val[0]));  // a segment is of one text
+            const uint32_t same = orderEqual(val, size, equal, [&](uint32_t x, uint32_t y) {
+                return directOrder(texts.packed, texts.bits, end, samplePosition(x), samplePosition(y), depth);
+            });
             uint64_t number = 0;
 #pragma unroll
             for (uint32_t i = 0; i < kSegTiny; i++) {
