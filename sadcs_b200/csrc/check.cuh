@@ -187,12 +187,15 @@ inline uint64_t inverseChunks(uint64_t n) {
 
 // Walks every piece. sorted: BWT positions in sorted order; starts[c]: the first sorted place of byte c
 // (256 entries). control[0]: pieces handed out, control[1]: chunks reserved (both zeroed by the
-// caller). jump[q] = the piece after piece q in the high word and q's length in the low one.
+// caller). jump[q] = the piece after piece q in the high word and q's length in the low one. gaveUp: the
+// sort's error word; where it is set, sorted is no permutation and a walk along it may never come to a
+// splitter, so every piece is left empty.
 __global__ void __launch_bounds__(kWalkThreads) inverseWalk(const uint32_t* __restrict__ sorted, uint32_t n,
                                                             uint32_t primary, const uint32_t* __restrict__ starts,
                                                             uint32_t pieces, uint32_t* __restrict__ control,
                                                             uint32_t maxChunks, uint4* __restrict__ chunks,
-                                                            uint2* __restrict__ owner, uint64_t* __restrict__ jump) {
+                                                            uint2* __restrict__ owner, uint64_t* __restrict__ jump,
+                                                            const uint32_t* __restrict__ gaveUp) {
     __shared__ uint32_t first[257];
     __shared__ uint8_t coarse[kCoarse];
     first[threadIdx.x] = starts[threadIdx.x];
@@ -233,8 +236,8 @@ __global__ void __launch_bounds__(kWalkThreads) inverseWalk(const uint32_t* __re
             if (piece > pieces) break;
             row = piece < pieces ? splitterRow(piece) : primary;
             length = 0;
-            if (row == 0 || row > n || (piece == pieces && row == splitterRow(row / kInverseStride))) {
-                // no such row, or the primary row is a splitter itself
+            if (row == 0 || row > n || *gaveUp || (piece == pieces && row == splitterRow(row / kInverseStride))) {
+                // no such row, no order to follow, or the primary row is a splitter itself
                 jump[piece] = static_cast<uint64_t>(piece == pieces ? row / kInverseStride : pieces + 1) << 32;
                 piece = kNoPiece;
                 continue;
@@ -445,7 +448,7 @@ inline cudaError_t inverseBwt(const uint8_t* bwt, uint32_t n, uint32_t primary, 
         ByteLoader{bwt}, ValueStorer{sorted, n}, ManySegments{tileStart, elementStart, segments}, n, ceilDiv(n, kSortTile),
         hist, radix, stream)));
     SADCS_TRY(launch(inverseWalk, inverseBlocks(n), kWalkThreads, 0, stream, sorted, n, primary, starts, pieces, control,
-                     maxChunks, chunkData, owner, jump[0]));
+                     maxChunks, chunkData, owner, jump[0], radix.control + 1));
     int cur = 0;
     for (uint64_t reach = 1; reach < static_cast<uint64_t>(pieces) + 2; reach *= 2, cur ^= 1) {
         SADCS_TRY(launch(inverseJump, ceilDiv(static_cast<uint64_t>(pieces) + 2, 256), 256, 0, stream, jump[cur],

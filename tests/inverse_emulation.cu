@@ -52,3 +52,40 @@ extern "C" int inverse_emulate(const uint8_t* bwt, int64_t n64, int64_t primary6
     }
     return jump[pieces] >> 32 == pieces + 1 && static_cast<uint32_t>(jump[pieces]) == n;
 }
+
+// On the GPU: the walk after a sort that gave up (its error word set). order: what the sort left (n
+// entries). Returns the characters walked, or -1 if a CUDA call failed; *chunks gets the chunks reserved.
+extern "C" int64_t inverse_walk_after_time_out(const uint32_t* order, int64_t n64, int64_t primary, int64_t* chunks) {
+    const uint32_t n = static_cast<uint32_t>(n64), pieces = inversePieces(n);
+    const uint64_t most = inverseChunks(n);
+    uint32_t *sorted = nullptr, *starts = nullptr, *control = nullptr;  // control[0..1], then the error word
+    uint4* data = nullptr;
+    uint2* owner = nullptr;
+    uint64_t* jump = nullptr;
+    std::vector<uint64_t> lengths(pieces + 2, 0);
+    const uint32_t words[4] = {0, 0, 1, 0};
+    uint32_t after[2] = {0, 0};
+    const bool ok = cudaMalloc(&sorted, 4 * static_cast<size_t>(n)) == cudaSuccess && cudaMalloc(&starts, 1024) == cudaSuccess &&
+                    cudaMalloc(&control, sizeof words) == cudaSuccess && cudaMalloc(&data, 16 * most) == cudaSuccess &&
+                    cudaMalloc(&owner, 8 * most) == cudaSuccess && cudaMalloc(&jump, 8 * lengths.size()) == cudaSuccess &&
+                    cudaMemcpy(sorted, order, 4 * static_cast<size_t>(n), cudaMemcpyHostToDevice) == cudaSuccess &&
+                    cudaMemset(starts, 0, 1024) == cudaSuccess &&
+                    cudaMemcpy(control, words, sizeof words, cudaMemcpyHostToDevice) == cudaSuccess &&
+                    launch(inverseWalk, inverseBlocks(n), kWalkThreads, 0, nullptr, sorted, n, static_cast<uint32_t>(primary),
+                           starts, pieces, control, static_cast<uint32_t>(most), data, owner, jump, control + 2) == cudaSuccess &&
+                    cudaDeviceSynchronize() == cudaSuccess &&
+                    cudaMemcpy(lengths.data(), jump, 8 * lengths.size(), cudaMemcpyDeviceToHost) == cudaSuccess &&
+                    cudaMemcpy(after, control, sizeof after, cudaMemcpyDeviceToHost) == cudaSuccess;
+    for (void* p : {static_cast<void*>(sorted), static_cast<void*>(starts), static_cast<void*>(control),
+                    static_cast<void*>(data), static_cast<void*>(owner), static_cast<void*>(jump)}) {
+        if (p) cudaFree(p);
+    }
+    if (!ok) return -1;
+    *chunks = after[1];
+    int64_t walked = 0;
+    for (uint64_t v : lengths) {
+        walked += static_cast<uint32_t>(v);
+        if (v >> 32 > pieces + 1) return -1;  // an entry that the jumps could not follow
+    }
+    return walked;
+}

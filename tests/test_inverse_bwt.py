@@ -45,6 +45,7 @@ def emulation():
                                         ctypes.byref(outside))
         return bool(valid), text, outside.value
 
+    run.library = library
     return run
 
 
@@ -170,3 +171,16 @@ def test_memory_beside_the_output(n, offset):
         except sa.GpuError:
             pass
         assert bool((margin[:offset] == 0xA5).all()) and bool((margin[offset + n:] == 0xA5).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 130, 100_000])
+def test_walk_after_a_sort_that_gave_up(n, emulation):
+    """The walk follows no order that its sort has not finished (every entry of this one leads to row 0)."""
+    order = np.zeros(n, np.uint32)
+    chunks = ctypes.c_int64(-1)
+    walk = emulation.library.inverse_walk_after_time_out
+    walk.restype = ctypes.c_int64
+    walk.argtypes = [ctypes.POINTER(ctypes.c_uint32), ctypes.c_int64, ctypes.c_int64, ctypes.POINTER(ctypes.c_int64)]
+    walked = walk(order.ctypes.data_as(ctypes.POINTER(ctypes.c_uint32)), n, 1, ctypes.byref(chunks))
+    assert walked == 0 and chunks.value == 0
