@@ -18,6 +18,10 @@
  *     calling thread is sadcs_gpu_last_error().
  *   - A context serves one thread at a time (gpusa.h:91); different threads use different contexts.
  *     Contexts are bound to the device that was current when they were created.
+ *   - The temporary device memory of the calls without a context (sadcs_gpu_check_*, sadcs_gpu_lcp,
+ *     sadcs_gpu_inverse_bwt, sadcs_gpu_bwt_from_sa) comes from one pool per device and process, which keeps up
+ *     to 2 GiB of it between calls. Other processes see that much less free memory;
+ *     sadcs_gpu_query_device gives all of it back.
  *
  * Extensions (marked "no counterpart"): 64-bit sizes with uint32 suffix arrays for texts of 2 GiB
  * and more (up to 2^32 - 256 bytes), SA and BWT from one construction, device-resident inputs and
@@ -85,7 +89,8 @@ int64_t sadcs_gpu_memory_reserve(void);
 /* gpuSampleSize, gpusa.h:57-60: sample positions (cover mod 32) in a text of n bytes. */
 int64_t sadcs_gpu_sample_size(int64_t n);
 
-/* gpuQueryDevice, gpusa.h:76: the current CUDA device and its memory. */
+/* gpuQueryDevice, gpusa.h:76: the current CUDA device and its memory. Temporary memory kept between calls
+ * (see above) is given back first, so this is also the call that frees it. */
 int sadcs_gpu_query_device(sadcs_gpu_device* device);
 
 /* gpuRequiredBytes, gpusa.h:79: peak device memory of a construction of n bytes, -1 if n is out of

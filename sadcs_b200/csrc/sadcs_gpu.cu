@@ -20,6 +20,7 @@
 #include <string>
 #include <vector>
 
+#include <cuda.h>
 #include <nvtx3/nvToolsExt.h>
 
 #include "alphabet.cuh"
@@ -338,21 +339,53 @@ void destroyContext(sadcs_gpu_context* c) {
 // does not map and unmap its memory each time (at 128 MiB the LCP array took 18-23 ms a call, 11 of
 // them on the device, with the default pool, which gives everything back at every
 // synchronisation). Whatever is kept is given back before free memory is reported (sadcs_gpu_query_device),
-// counted for a server, or found too little for a context. The pool itself is safe across threads and
-// streams.
+// counted for a server, or found too little for a context; the driver also takes a pool's unused memory for any
+// other allocation of the process that would fail without it. The pool itself is safe across threads
+// and streams. It outlives cudaDeviceReset, but what it holds belongs to the context that is gone, so it is
+// replaced when the context is another one.
 constexpr uint64_t kWorkspaceKeep = uint64_t(2) << 30;
 constexpr int kWorkspaceDevices = 64;
+struct WorkspacePool {
+    cudaMemPool_t pool = nullptr;
+    unsigned long long context = 0;  // of the pool's allocations
+};
 std::mutex gWorkspaceLock;
-cudaMemPool_t gWorkspacePool[kWorkspaceDevices] = {};
+WorkspacePool gWorkspacePool[kWorkspaceDevices];
 
-cudaError_t workspacePool(cudaMemPool_t* pool, bool create) {
-    *pool = nullptr;
+// The current context's number, never given to two contexts of a process.
+cudaError_t contextNumber(unsigned long long* number) {
+    using GetId = CUresult(CUDAAPI*)(CUcontext, unsigned long long*);
+    static const GetId getId = [] {
+        void* entry = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const cudaError_t error = cudaGetDriverEntryPointByVersion("cuCtxGetId", &entry, 12000, cudaEnableDefault, &found);
+        return error == cudaSuccess && found == cudaDriverEntryPointSuccess ? reinterpret_cast<GetId>(entry) : nullptr;
+    }();
+    const cudaError_t error = cudaFree(nullptr);  // makes the device's context current if there is none
+    if (error != cudaSuccess) return error;
+    if (!getId) return cudaErrorNotSupported;
+    return getId(nullptr, number) == CUDA_SUCCESS ? cudaSuccess : cudaErrorDeviceUninitialized;
+}
+
+// Runs use(pool) on the current device's pool, which no other thread replaces meanwhile; without a pool
+// (create false) nothing.
+template <class Use>
+cudaError_t withWorkspacePool(bool create, Use use) {
     int device = 0;
+    unsigned long long context = 0;
     cudaError_t error = cudaGetDevice(&device);
     if (error != cudaSuccess) return error;
     if (device < 0 || device >= kWorkspaceDevices) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> hold(gWorkspaceLock);
-    if (!gWorkspacePool[device] && create) {
+    WorkspacePool& w = gWorkspacePool[device];
+    if (!w.pool && !create) return cudaSuccess;
+    if ((error = contextNumber(&context)) != cudaSuccess) return error;
+    if (w.pool && w.context != context) {
+        cudaMemPoolDestroy(w.pool);  // at once, or with the last allocation that another context still uses
+        w.pool = nullptr;
+        if (!create) return cudaSuccess;
+    }
+    if (!w.pool) {
         cudaMemPoolProps props = {};
         props.allocType = cudaMemAllocationTypePinned;
         props.handleTypes = cudaMemHandleTypeNone;
@@ -365,24 +398,22 @@ cudaError_t workspacePool(cudaMemPool_t* pool, bool create) {
             cudaMemPoolDestroy(made);
             return error;
         }
-        gWorkspacePool[device] = made;
+        w.pool = made;
+        w.context = context;
     }
-    *pool = gWorkspacePool[device];
-    return cudaSuccess;
+    return use(w.pool);
 }
 
 // Device memory from the pool, in stream order (freed with cudaFreeAsync).
 template <class T>
 cudaError_t workspace(T** memory, size_t bytes, cudaStream_t stream) {
-    cudaMemPool_t pool = nullptr;
-    const cudaError_t error = workspacePool(&pool, true);
-    if (error != cudaSuccess) return error;
-    return cudaMallocFromPoolAsync(reinterpret_cast<void**>(memory), bytes, pool, stream);
+    return withWorkspacePool(true, [&](cudaMemPool_t pool) {
+        return cudaMallocFromPoolAsync(reinterpret_cast<void**>(memory), bytes, pool, stream);
+    });
 }
 
 void trimWorkspace() {
-    cudaMemPool_t pool = nullptr;
-    if (workspacePool(&pool, false) == cudaSuccess && pool) cudaMemPoolTrimTo(pool, 0);
+    withWorkspacePool(false, [](cudaMemPool_t pool) { return cudaMemPoolTrimTo(pool, 0); });
 }
 
 // giveBack: the workspace pool's unused memory goes back first, so that it counts as free.
