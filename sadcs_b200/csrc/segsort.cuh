@@ -223,7 +223,24 @@ __global__ void __launch_bounds__(256) segDigitBase(uint32_t* __restrict__ hist,
 #ifndef SADCS_DIRECT_WORDS
 #define SADCS_DIRECT_WORDS 8
 #endif
-constexpr uint32_t kDirectList = 8u << 20;
+#ifndef SADCS_DIRECT_LIST
+#define SADCS_DIRECT_LIST (8u << 20)
+#endif
+constexpr uint32_t kDirectList = SADCS_DIRECT_LIST;
+// Direct where at least 1 of kDirectShare elements in the sample (one block in kDirectSample) was decided.
+// Ranking of a text and one copy of it with point changes, without direct comparisons, with them in every pass, and
+// by the rule: 192 MiB of 2-bit codes, changes at 0.2% (40% of the pairs decided) 44.2, 36.7, 36.5 ms, 0.8% 28.8,
+// 17.9, 17.8; three copies of 96 MiB of bytes, 0.4% (23%) 42.3, 52.8, 42.4, 0.8% (40%) 36.6, 40.1, 36.7, 1.6%
+// 30.8, 27.3, 25.3; exact copies of it 144.5, 148.3, 144.6. With 1 in 2 and 1 in 3 some of the gains are left, with
+// 1 in 6 the next rate's are had too; none of them costs more than 0.3% anywhere.
+#ifndef SADCS_DIRECT_SHARE
+#define SADCS_DIRECT_SHARE 4
+#endif
+constexpr uint32_t kDirectShare = SADCS_DIRECT_SHARE;
+constexpr uint32_t kDirectSample = 64;
+__host__ __device__ __forceinline__ bool directWorthwhile(uint32_t compared, uint32_t decided) {
+    return static_cast<uint64_t>(decided) * kDirectShare >= compared;
+}
 __host__ __device__ __noinline__ int directOrder(const uint64_t* __restrict__ packed, uint32_t b, uint32_t end, uint32_t i,
                                                  uint32_t j, uint32_t from) {
     const uint32_t perWord = 64 / b, shorter = end - (i > j ? i : j);  // characters of the shorter suffix
@@ -273,13 +290,26 @@ __host__ __device__ __forceinline__ uint32_t orderEqual(uint32_t (&val)[kSegTiny
 // genome-like text most groups left after the first pass are a repeat and its copies (2-4 members),
 // which agree for about a hundred characters. A sorted segment's keys are replaced by
 // numbers that differ where the order is known, so members that still agree stay a group, which
-// shares `depth` characters as every group of the pass does. tied counts the elements compared directly.
-// Written back in place.
+// shares `depth` characters as every group of the pass does. Written back in place.
+// Whole copies agree for far longer, and comparing them would only repeat itself in every pass. So one block
+// in kDirectSample goes first (sampled) and counts what it compared and decided in direct[0] and [1]; the
+// others compare if that share was worth it. direct[2] counts all elements decided this way.
 template <bool kDirect>
 __global__ void __launch_bounds__(256) segSortTiny(const uint32_t* __restrict__ heads, uint32_t segments, TextSet texts,
                                                    uint32_t depth, uint64_t* __restrict__ keys,
-                                                   uint32_t* __restrict__ vals, uint32_t* __restrict__ tied) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+                                                   uint32_t* __restrict__ vals, uint32_t* __restrict__ direct, bool sampled) {
+    uint32_t block = blockIdx.x;
+    bool compare = false;
+    if constexpr (kDirect) {
+        if (sampled) {
+            block *= kDirectSample;
+            compare = true;
+        } else {
+            if (block % kDirectSample == 0) return;
+            compare = directWorthwhile(direct[0], direct[1]);
+        }
+    }
+    const uint32_t k = block * blockDim.x + threadIdx.x;
     if (k >= segments) return;
     const uint32_t begin = heads[k], size = heads[k + 1] - begin;
     if (size < 2 || size > kSegTiny) return;
@@ -314,12 +344,17 @@ __global__ void __launch_bounds__(256) segSortTiny(const uint32_t* __restrict__ 
         for (uint32_t i = 0; i + 1 < kSegTiny; i++) {
             if (i + 1 < size && key[i] == key[i + 1]) equal |= 1u << i;
         }
-        if (equal) {
-            atomicAdd(tied, static_cast<uint32_t>(__popc(equal | (equal << 1))));
+        if (equal && compare) {
             const uint32_t end = texts.endOf(samplePosition(val[0]));  // a segment is of one text
             const uint32_t same = orderEqual(val, size, equal, [&](uint32_t x, uint32_t y) {
                 return directOrder(texts.packed, texts.bits, end, samplePosition(x), samplePosition(y), depth);
             });
+            const uint32_t compared = equal | (equal << 1), decided = compared & ~(same | (same << 1));
+            if (sampled) {
+                atomicAdd(direct, static_cast<uint32_t>(__popc(compared)));
+                atomicAdd(direct + 1, static_cast<uint32_t>(__popc(decided)));
+            }
+            if (decided) atomicAdd(direct + 2, static_cast<uint32_t>(__popc(decided)));
             uint64_t number = 0;
 #pragma unroll
             for (uint32_t i = 0; i < kSegTiny; i++) {
@@ -539,9 +574,10 @@ struct SegBuffers {
     uint32_t* perSeg;   // 2 * u words (free key buffer): big flags and tile counts per segment
     uint32_t* scratch;  // scratchWords words, at least segScratchWords(u)
     size_t scratchWords;
-    uint32_t* counter;  // device words [0..3]; [3]: elements that segSortTiny compared directly
+    uint32_t* counter;  // device words [0..5]; [3..5]: segSortTiny<true>'s counts
     uint32_t* scanScratch;
-    bool* compared;     // (host) set when segSortTiny<true> ran: counter[3] holds its count
+    bool direct;        // (host) whether elements of equal keys may be compared directly
+    bool* compared;     // (host) set when segSortTiny<true> ran: counter[3..5] hold its counts
 };
 
 // Sorts the list (keys, vals: u elements, compact sample indices, in segments of equal grp) by key inside
@@ -590,16 +626,20 @@ inline cudaError_t segmentedSort(const uint32_t* grp, uint32_t u, uint64_t* keys
     // triples: 2 GiB of genome-like text (59M samples listed, groups of 2.2) ranks in 49.8 ms against
     // 58.2, five doubling rounds fewer; elsewhere they are made again in every pass for groups that
     // stay (48 MiB of versions of one document, groups of 48: 15.9 ms against 13.5) or come on top of the
-    // passes that larger groups need anyway (256 MiB of natural-language-like text: 17.3 against 16.9).
-    const bool direct = u >= kDirectList && u <= 3 * static_cast<uint64_t>(segments);
+    // passes that larger groups need anyway (256 MiB of natural-language-like text: 17.3 against 16.9). Whether
+    // the pairs and triples agree for too long is found by a sample (kDirectShare).
+    const bool direct = b.direct && u >= kDirectList && u <= 3 * static_cast<uint64_t>(segments);
     if (direct) {
         *b.compared = true;
-        SADCS_TRY(cudaMemsetAsync(b.counter + 3, 0, sizeof(uint32_t), stream));
-        SADCS_TRY(launch(segSortTiny<true>, ceilDiv(segments, 256), 256, 0, stream, b.heads, segments, texts, depth, keys,
-                         vals, b.counter + 3));
+        SADCS_TRY(cudaMemsetAsync(b.counter + 3, 0, 3 * sizeof(uint32_t), stream));
+        const uint32_t blocks = ceilDiv(segments, 256);
+        SADCS_TRY(launch(segSortTiny<true>, ceilDiv(blocks, kDirectSample), 256, 0, stream, b.heads, segments, texts, depth,
+                         keys, vals, b.counter + 3, true));
+        SADCS_TRY(launch(segSortTiny<true>, blocks, 256, 0, stream, b.heads, segments, texts, depth, keys, vals,
+                         b.counter + 3, false));
     } else {
         SADCS_TRY(launch(segSortTiny<false>, ceilDiv(segments, 256), 256, 0, stream, b.heads, segments, texts, depth, keys,
-                         vals, b.counter + 3));
+                         vals, b.counter + 3, false));
     }
     SADCS_TRY(launch(segSortSmall, ceilDiv(u, kSegChunk), kSegThreads, segSortSharedBytes(), stream, b.heads,
                      segments, keys, vals, keys, vals, keyBits));

@@ -5,8 +5,11 @@ the direct comparison, and a copy that ends with the text. The CPU tests run the
 by it (tests/direct_emulation.cu, built with nvcc) on groups of every size."""
 import ctypes
 import itertools
+import os
+import re
 import shutil
 import subprocess
+import sys
 from pathlib import Path
 
 import numpy as np
@@ -146,3 +149,43 @@ def test_repeats(sigma, n):
     out = torch.empty_like(text)
     sa.inverse_bwt_device(bwt.data_ptr(), n, primary, out.data_ptr())
     assert torch.equal(out, text)
+
+
+TRACED = """
+import sys
+import torch
+import sadcs_b200 as sa
+
+sigma, copies, rate = int(sys.argv[1]), int(sys.argv[2]), float(sys.argv[3])
+n = 32 << 20
+g = torch.Generator(device="cuda").manual_seed(sigma)
+x = torch.randint(0, sigma, (n,), dtype=torch.uint8, device="cuda", generator=g)
+parts = [x]
+for _ in range(copies):
+    changed = torch.rand(n, device="cuda", generator=g) < rate
+    parts.append(torch.where(changed, torch.randint(0, sigma, (n,), dtype=torch.uint8, device="cuda", generator=g), x))
+text = torch.cat(parts)
+out = torch.empty(text.numel(), dtype=torch.int32, device="cuda")
+torch.cuda.synchronize()
+sa.build_device(text.data_ptr(), text.numel(), out.data_ptr(), None)
+assert sa.check_suffix_array_device(text.data_ptr(), text.numel(), out.data_ptr()) == (True, -1, None)
+"""
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sigma,copies,rate,passes", [(4, 1, 0.0, 1), (256, 2, 0.0, 1), (4, 1, 0.02, 1), (256, 1, 0.03, 1)])
+def test_direct_comparison_is_tried_and_left(sigma, copies, rate, passes):
+    """A text and copies of it: with changes the sample is decided and so are the groups; exact copies are sampled in
+    one pass, not compared beyond the sample, and not sampled again."""
+    done = subprocess.run([sys.executable, "-c", TRACED, str(sigma), str(copies), str(rate)], capture_output=True,
+                          text=True, cwd=HERE.parent, env={**os.environ, "SADCS_TRACE": "1"}, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
+    found = [tuple(map(int, m)) for m in re.findall(
+        r"direct comparison decided (\d+) of (\d+) sampled, (\d+) in all", done.stderr)]
+    assert len(found) == passes, done.stderr
+    decided, sampled, total = found[0]
+    assert sampled > 0
+    if rate:
+        assert 4 * decided >= sampled and total > 32 * decided
+    else:
+        assert decided == 0 and total == 0
