@@ -152,56 +152,47 @@ __global__ void segCollectBig(const uint32_t* __restrict__ heads, uint32_t segme
 }
 
 // hist[(p * segments + s) * 256 + digit] of digit passes first .. first + passes - 1 (bits [8q, 8q + 8) of
-// pass q) of every big segment s (zeroed by the caller). A block takes kHistTiles tiles and keeps one
-// shared histogram per pass for as long as they are of one segment. All passes are counted from one
+// pass q) of every big segment s (zeroed by the caller), one tile per block. All passes are counted from one
 // read of the keys where their tables fit the scratch: the 4096-text batch's first sort spent 6.5 ms
 // of 45 on reading its keys once per pass. Runs of equal digits are counted in registers and added to
-// the shared histogram when the digit changes, as in radixHistogramFrom.
-constexpr uint32_t kHistTiles = 4;
-__global__ void __launch_bounds__(256) segHistogram(const uint64_t* __restrict__ keys, ListSegments segs,
-                                                    uint32_t tiles, int firstPass, int passes,
-                                                    uint32_t* __restrict__ hist) {
+// the shared histogram when the digit changes, as in radixHistogramFrom. Four tiles per block, whose counts
+// go out once per segment, gain the batch nothing (74.5 ms of ranking both ways) and leave smaller lists too
+// few blocks (a run of 32 MiB of one character 13.9 ms, 13.5 with one).
+__global__ void __launch_bounds__(256) segHistogram(const uint64_t* __restrict__ keys, ListSegments segs, int firstPass,
+                                                    int passes, uint32_t* __restrict__ hist) {
     __shared__ uint32_t h[8][256];
     for (int p = 0; p < passes; p++) h[p][threadIdx.x] = 0;
     __syncthreads();
-    const uint32_t firstTile = blockIdx.x * kHistTiles, endTile = min(firstTile + kHistTiles, tiles);
-    for (uint32_t t = firstTile; t < endTile; t++) {
-        uint32_t segment, segTile, begin, size;
-        segs.locate(t, segment, segTile, begin, size);
-        const uint32_t local = t - segTile;
-        const uint32_t tileEnd = min((local + 1) * kSortTile, size);
-        uint32_t run[8], digit[8];
+    uint32_t segment, segTile, begin, size;
+    segs.locate(blockIdx.x, segment, segTile, begin, size);
+    const uint32_t local = blockIdx.x - segTile;
+    const uint32_t tileEnd = min((local + 1) * kSortTile, size);
+    uint32_t run[8], digit[8];
 #pragma unroll
-        for (int p = 0; p < 8; p++) run[p] = digit[p] = 0;
-        for (uint32_t k = local * kSortTile + threadIdx.x; k < tileEnd; k += blockDim.x) {
-            const uint64_t key = keys[begin + k] >> (8 * firstPass);
-#pragma unroll
-            for (int p = 0; p < 8; p++) {
-                if (p < passes) {
-                    const uint32_t d = static_cast<uint32_t>(key >> (8 * p)) & 0xFF;
-                    if (d != digit[p]) {
-                        if (run[p]) atomicAdd(&h[p][digit[p]], run[p]);
-                        digit[p] = d;
-                        run[p] = 0;
-                    }
-                    run[p]++;
-                }
-            }
-        }
+    for (int p = 0; p < 8; p++) run[p] = digit[p] = 0;
+    for (uint32_t k = local * kSortTile + threadIdx.x; k < tileEnd; k += blockDim.x) {
+        const uint64_t key = keys[begin + k] >> (8 * firstPass);
 #pragma unroll
         for (int p = 0; p < 8; p++) {
-            if (p < passes && run[p]) atomicAdd(&h[p][digit[p]], run[p]);
-        }
-        // the last tile of the block or of its segment: the counts go out
-        if (t + 1 == endTile || tileEnd == size) {
-            __syncthreads();
-            for (int p = 0; p < passes; p++) {
-                const uint32_t c = h[p][threadIdx.x];
-                if (c) atomicAdd(hist + (static_cast<size_t>(p) * segs.segments + segment) * 256 + threadIdx.x, c);
-                h[p][threadIdx.x] = 0;
+            if (p < passes) {
+                const uint32_t d = static_cast<uint32_t>(key >> (8 * p)) & 0xFF;
+                if (d != digit[p]) {
+                    if (run[p]) atomicAdd(&h[p][digit[p]], run[p]);
+                    digit[p] = d;
+                    run[p] = 0;
+                }
+                run[p]++;
             }
-            __syncthreads();
         }
+    }
+#pragma unroll
+    for (int p = 0; p < 8; p++) {
+        if (p < passes && run[p]) atomicAdd(&h[p][digit[p]], run[p]);
+    }
+    __syncthreads();
+    for (int p = 0; p < passes; p++) {
+        const uint32_t c = h[p][threadIdx.x];
+        if (c) atomicAdd(hist + (static_cast<size_t>(p) * segs.segments + segment) * 256 + threadIdx.x, c);
     }
 }
 
@@ -667,8 +658,7 @@ inline cudaError_t segmentedSort(const uint32_t* grp, uint32_t u, uint64_t* keys
     for (int p = 0; p < passes; p++) {
         if (p % together == 0) {
             SADCS_TRY(cudaMemsetAsync(hist, 0, together * table * 4, stream));
-            SADCS_TRY(launch(segHistogram, ceilDiv(bigTiles, kHistTiles), 256, 0, stream, kIn, segs, bigTiles, p,
-                             together, hist));
+            SADCS_TRY(launch(segHistogram, bigTiles, 256, 0, stream, kIn, segs, p, together, hist));
             SADCS_TRY(launch(segDigitBase, big * together, 256, 0, stream, hist, begin, big));
         }
         SortLoader<uint64_t> ld{kIn, vIn, 8 * p};
