@@ -107,6 +107,15 @@ __device__ __forceinline__ uint32_t classOfResidue(uint32_t r) {
     return static_cast<uint32_t>(__ffs(__funnelshift_r(kCoverMask, kCoverMask, r))) - 1;
 }
 
+inline int bitWidth(uint64_t x) {
+    int b = 0;
+    while (x) {
+        b++;
+        x >>= 1;
+    }
+    return b;
+}
+
 inline uint64_t sampleSize(uint64_t n) {
     return n == 0 ? 0 : packHost(n);
 }

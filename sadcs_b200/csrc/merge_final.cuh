@@ -480,17 +480,31 @@ inline cudaError_t launchTreeWidth(const MergeArgs& args, uint32_t tiles, cudaSt
     }
 }
 
-// Whether a construction merges with merge_wide.cuh's kernel. deep: the samples that still shared
-// their first 20 characters or more with another (RankStats). That kernel compares a few words per
-// record cheaply and puts records that agree in all of them in order afterwards, one tile phase more;
-// this one decides such ties where they are met. Final level with few ties (deep = 0): the
-// 4096-text batch 69.0 ms against 130.8 here, 100 MB of protein-like text 2.39 against 3.03, 8 MiB of
-// uniform bytes 0.213 against 0.303; with many: 256 MiB of natural-language-like text (a third of
-// its samples deep) 17.3 against 14.95, 48 MiB of versions of one document 6.0 against 2.1. The
-// narrow codes' one-word records (a key alone) gain nothing and lose on repeats (2 GiB of genome-like
-// text 58-70 ms against 48.2), so they stay here.
-inline bool useWideMerge(uint32_t bits, uint64_t deep, uint64_t samples) {
-    return finalWords(bits) > 1 && deep <= samples / 32;
+// The characters that merge_wide.cuh's kernel can tell a tile's records apart by, for `outputs` characters in
+// codes of `bits` bits: the 112 bits it holds of a record and the bits that a tile's records share, about
+// log2 of the number of tiles where the text does not repeat itself.
+inline uint64_t wideMergeChars(uint32_t bits, uint64_t outputs) {
+    return (112 + bitWidth(outputs / mergeCap(kWideR))) / bits;
+}
+
+// Whether a construction merges with merge_wide.cuh's kernel. ties: its samples that share wideMergeChars or
+// more with another. That kernel compares a few words per record cheaply and puts records that agree in all of
+// them in order afterwards, one tile phase more; this one holds more words the wider the codes are and decides
+// ties where they are met. Final level without ties: the 4096-text batch 69.0 ms against 130.8 here, 100 MB of
+// protein-like text 2.39 against 3.03, 8 MiB of uniform bytes 0.213 against 0.303. With ties, 64 MiB of random
+// text of which a share is repeats of 13 to 1000 characters, each 2 or 16 times, merge in all (wide / here):
+//   words (bits)   no ties      up to the line   above it
+//   2 (3, 4)       0.92         0.95 - 1.00      0.94 - 1.14 at up to 1 in 32, then 0.96 - 1.5
+//   3 (5, 6)       0.83         0.85 - 1.08      0.88 - 1.26 at up to 1 in 32, then 0.89 - 1.8
+//   4 (7, 8)       0.70 - 0.72  0.73 - 0.99      0.75 - 1.25 at up to 1 in 16, then 0.84 - 1.9
+// (the count is of samples tied with samples, so repeats of two count for less than they cost). The line lies where the
+// dearest of the repeats measured come to this kernel's time; 48 MiB of versions of one document, nearly all
+// tied, take 6.0 against 2.1, 256 MiB of natural-language-like text, a third, 17.3 against 14.95. One-word
+// records (2-bit codes, a key alone) gain nothing and lose on repeats (2 GiB of genome-like text 58-70 ms
+// against 48.2), so they stay here.
+inline bool useWideMerge(uint32_t bits, uint64_t ties, uint64_t samples) {
+    const int words = finalWords(bits);
+    return words > 1 && ties <= samples >> (9 - words);
 }
 
 // One merge level: kFinal writes the SA and BWT, otherwise the rows of the level below.

@@ -421,15 +421,6 @@ inline uint32_t blocks256(uint64_t count) {
     return static_cast<uint32_t>((count + 255) / 256);
 }
 
-inline int bitWidth(uint64_t x) {
-    int b = 0;
-    while (x) {
-        b++;
-        x >>= 1;
-    }
-    return b;
-}
-
 // Characters of the first character pass of one text, a global sort of every sample: the fewest
 // whole 8-bit radix passes whose key, tag included, holds enough characters for 2^(chars * bits)
 // to exceed 16 times the samples (on a text without repeats, about 1 sample in 16 then shares its
@@ -463,22 +454,39 @@ inline uint32_t firstPassChars(const TextSet& texts, uint64_t samples) {
     return texts.keyChars;
 }
 
-constexpr uint64_t kDeepChars = 20;
+// How many samples share at least a given number of characters with another one, from the lists left
+// by the passes: those on either side of that depth, interpolated.
+struct TieCount {
+    uint64_t chars;             // the depth asked for
+    uint64_t depth = 0, count;  // of the last pass noted
+    bool known = false;
+    TieCount(uint64_t charsAsked, uint64_t live) : chars(charsAsked), count(live) {}
+    // A pass that reached `reached` characters left `left` samples that share them.
+    void note(uint64_t reached, uint64_t left) {
+        if (known) return;
+        if (reached >= chars) {
+            known = true;
+            left = count - (count - std::min(left, count)) * (chars - depth) / (reached - depth);
+        }
+        depth = reached;
+        count = left;
+    }
+};
+
 struct RankStats {
     int characterPasses = 0;
     int doublingRounds = 0;
-    // Samples that shared about kDeepChars characters or more with another: those still listed after the
-    // pass that reached them and those compared directly until then.
-    uint64_t deep = 0;
+    uint64_t ties = 0;  // samples that share at least tieChars characters with another (TieCount)
 };
 
 // Ranks the live sample suffixes of the texts. slots = rank entries (sample positions of the whole
 // concatenation); live = live samples; sampleBase (device, per text) is used with several texts.
 // Ranks of live samples end up in [0, live), text by text; ranks are zeroed by the caller for one
-// text (and kRankPad entries past slots always). hostCounter: page-locked words (11).
+// text (and kRankPad entries past slots always). hostCounter: page-locked words (11). tieChars: the depth at
+// which ties are counted.
 inline cudaError_t rankSample(const uint8_t* text, const TextSet& texts, uint32_t slots, uint32_t live,
                               const uint32_t* sampleBase, uint32_t longest, uint32_t* ranks, RankBuffers b,
-                              uint32_t* hostCounter, cudaStream_t stream, RankStats& stats) {
+                              uint32_t* hostCounter, cudaStream_t stream, uint64_t tieChars, RankStats& stats) {
     if (live == 0) return cudaSuccess;
     uint32_t* cur = b.lst[0];
     uint32_t* alt = b.lst[1];
@@ -489,7 +497,8 @@ inline cudaError_t rankSample(const uint8_t* text, const TextSet& texts, uint32_
     SADCS_TRY(cudaMemsetAsync(error, 0, sizeof(uint32_t), stream));
     uint32_t u = live;
     uint64_t depth = 0, direct = 0;
-    bool deepKnown = false, tryDirect = true;
+    bool tryDirect = true;
+    TieCount ties(tieChars, live);
     bool first = texts.count <= 1;  // one text: everything starts in one group, no group sort
     const int rankBits = bitWidth(static_cast<uint64_t>(live) + 1);
     // The first pass of one text may key fewer characters (fewer radix passes over every sample).
@@ -584,11 +593,9 @@ inline cudaError_t rankSample(const uint8_t* text, const TextSet& texts, uint32_
             stats.characterPasses++;
             depth += passTexts.keyChars;
         }
-        if (!deepKnown) {
-            if (compared) direct += hostCounter[4];
-            stats.deep = u + direct;
-            deepKnown = depth >= kDeepChars;
-        }
+        if (compared) direct += hostCounter[4];
+        ties.note(depth, u + direct);
+        stats.ties = ties.count;
         first = false;
     }
     return cudaSuccess;

@@ -754,8 +754,8 @@ int construct(sadcs_gpu_context* c, const Batch& b, Io& io, cudaStream_t stream,
     rb.keyEntries = static_cast<uint32_t>(std::min(L.key1 - L.key0, L.grp - L.key1) / 8);
     RankStats rankStats;
     if ((error = rankSample(text, texts, static_cast<uint32_t>(b.slots), static_cast<uint32_t>(b.live), dSampleBase,
-                            static_cast<uint32_t>(b.longest), ranks, rb, c->hostWords, stream, rankStats)) !=
-        cudaSuccess) {
+                            static_cast<uint32_t>(b.longest), ranks, rb, c->hostWords, stream,
+                            wideMergeChars(texts.bits, b.outputs), rankStats)) != cudaSuccess) {
         return failed("sample ranking", error);
     }
     s.character_passes = rankStats.characterPasses;
@@ -798,7 +798,11 @@ int construct(sadcs_gpu_context* c, const Batch& b, Io& io, cudaStream_t stream,
                             : (io.outSa ? io.outSa : (io.wantSa ? reinterpret_cast<uint32_t*>(slab + L.sa) : nullptr));
     uint8_t* bwt = bwtPieces ? nullptr : (io.outBwt ? io.outBwt : (io.wantBwt ? slab + L.bwt : nullptr));
     // The merge's kernel and tile shape follow the code width and the ties, known now (the memory plan bounds every shape).
-    const bool wide = useWideMerge(texts.bits, rankStats.deep, b.live);
+    const bool wide = useWideMerge(texts.bits, rankStats.ties, b.live);
+    if (traceEnabled()) {
+        fprintf(stderr, "sadcs: merge %s, %llu of %llu samples tied\n", wide ? "wide" : "tree",
+                static_cast<unsigned long long>(rankStats.ties), static_cast<unsigned long long>(b.live));
+    }
     const MergePlan mergePlan = planMerge(b.classes.start, wide ? kWideR : mergeR(finalWords(texts.bits)));
     OverlappedDownload download;
     const bool overlapped = (io.hostSa || io.hostBwt) && c->copyStream;
@@ -1648,7 +1652,7 @@ int sadcs_gpu_rank_sample(const uint8_t* text, int64_t n, uint32_t* ranks, sadcs
         RankStats rankStats;
         if ((error = rankSample(textBuffer, texts, static_cast<uint32_t>(b.slots), static_cast<uint32_t>(b.live),
                                 nullptr, static_cast<uint32_t>(length), rankBuffer, rb, c->hostWords, c->stream,
-                                rankStats)) != cudaSuccess) {
+                                /*tieChars=*/0, rankStats)) != cudaSuccess) {
             return failed("sample ranking", error);
         }
         s.character_passes = rankStats.characterPasses;

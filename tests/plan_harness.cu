@@ -82,3 +82,13 @@ extern "C" uint64_t plan_tile_bound(const uint32_t* row, const uint32_t* start) 
     for (int b = 0; b < kClasses; b++) r.c[b] = row[1 + b];
     return tileOutputBound(r, start);
 }
+
+// The ties counted at `chars` characters from passes that reached depth[k] and left left[k] of `live` samples.
+extern "C" uint64_t tie_count(uint64_t chars, uint64_t live, const uint64_t* depth, const uint64_t* left, uint32_t passes) {
+    TieCount ties(chars, live);
+    for (uint32_t k = 0; k < passes; k++) ties.note(depth[k], left[k]);
+    return ties.count;
+}
+
+extern "C" int wide_merge(uint32_t bits, uint64_t ties, uint64_t samples) { return useWideMerge(bits, ties, samples); }
+extern "C" uint64_t wide_merge_chars(uint32_t bits, uint64_t outputs) { return wideMergeChars(bits, outputs); }
