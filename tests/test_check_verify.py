@@ -26,8 +26,11 @@ def _lcp_of_neighbours(text, suffixes, limit=64):
     return out
 
 
-@pytest.mark.parametrize("n", [257, 100_000, SLICED - 1, SLICED, SLICED + 4097])
-def test_verdicts(n):
+@pytest.mark.parametrize("n,full", [(257, False), (100_000, False), (SLICED - 1, False), (SLICED, False),
+                                    (SLICED + 4097, False), (SLICED, True), (SLICED + 4097, True)])
+def test_verdicts(n, full):
+    """full: the device's memory is filled until the pairs of the sliced writes (8n bytes) are not to be had and the
+    inverse and the LCP array's Phi (4n) are."""
     import torch
 
     g = torch.Generator(device="cuda").manual_seed(n)
@@ -40,11 +43,28 @@ def test_verdicts(n):
         torch.cuda.synchronize()
         return sa.check_suffix_array_device(text.data_ptr(), n, suffixes.data_ptr())
 
-    assert check() == (True, -1, None)
     lcp = torch.empty_like(suffixes)
+    correct = suffixes.clone()
+    if full:
+        check(), sa.lcp_device(text.data_ptr(), n, suffixes.data_ptr(), lcp.data_ptr())  # the kernels are loaded
+        expected_lcp = _lcp_of_neighbours(text, suffixes.to(torch.int64))
+        torch.cuda.empty_cache()
+        sa.query_device()
+        leave = 8 * n  # the check takes 4n, then 8n; the LCP array 12.13n, then 4.13n
+        filler = torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda")
+        assert 5 * n < torch.cuda.mem_get_info()[0] <= leave
+        assert check() == (True, -1, None)
+        sa.lcp_device(text.data_ptr(), n, suffixes.data_ptr(), lcp.data_ptr())
+        suffixes[n // 2] = correct[n // 3]
+        verdict = check()
+        suffixes.copy_(correct)
+        del filler
+        torch.cuda.empty_cache()
+        assert torch.equal(lcp.to(torch.int64), expected_lcp)
+        assert verdict == (False, n // 3, "duplicate entry")
+    assert check() == (True, -1, None)  # no error is left over
     sa.lcp_device(text.data_ptr(), n, suffixes.data_ptr(), lcp.data_ptr())
     assert torch.equal(lcp.to(torch.int64), _lcp_of_neighbours(text, suffixes.to(torch.int64)))
-    correct = suffixes.clone()
     i, j = n // 3, n - 2
     suffixes[[i, i + 1]] = correct[[i + 1, i]]  # neighbours exchanged: the pair itself or one beside it
     ok, index, reason = check()

@@ -1,6 +1,6 @@
 """The calls that keep temporary device memory between calls, before and after cudaDeviceReset: the same
-results, and what was kept under the context that is gone is given back. tests/reset_harness.cu (the library's
-source included whole, built with nvcc) runs in a process of its own, whose device state the reset ends."""
+results, and what was kept under the context that is gone is given back. tests/workspace_harness.cu (the
+library's source included whole, built with nvcc) runs in a process of its own, whose device state the reset ends."""
 import ctypes
 import json
 import shutil
@@ -11,9 +11,9 @@ from pathlib import Path
 import pytest
 
 HERE = Path(__file__).resolve().parent
-SOURCE = HERE / "reset_harness.cu"
+SOURCE = HERE / "workspace_harness.cu"
 CSRC = HERE.parent / "sadcs_b200" / "csrc"
-BUILT = HERE / "_build" / "libreset_harness.so"
+BUILT = HERE / "_build" / "libworkspace_harness.so"
 
 # A run of one character: its suffix array and LCP array are known, and the calls keep memory (12n bytes).
 CHILD = """
@@ -38,7 +38,7 @@ def harness():
     if not BUILT.exists() or BUILT.stat().st_mtime < newest:
         nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
         if not Path(nvcc).exists():
-            pytest.skip("nvcc is needed to build the reset harness")
+            pytest.skip("nvcc is needed to build the workspace harness")
         BUILT.parent.mkdir(exist_ok=True)
         tmp = BUILT.with_suffix(".so.tmp")
         subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O2", "-Xcompiler", "-fPIC",

@@ -2,12 +2,15 @@
 sadcs_gpu_check_suffix_array on the same device buffers: every verdict (ok, first failing index,
 reason) must agree, on two calls in a row, so scratch left by one call cannot change the next one's
 answer. This file sorts last so that it also runs after every other GPU test in one session."""
+import ctypes
+
 import numpy as np
 import pytest
 
 import oracle
 import sadcs_b200 as sa
 from sadcs_b200 import workloads as W
+from tests.test_device_reset import harness
 
 pytestmark = pytest.mark.gpu
 
@@ -103,3 +106,17 @@ def test_a_call_allocates_nothing():
     for _ in range(2):
         assert sa.check_suffix_array_static_device(d_text.data_ptr(), len(text), d_sa.data_ptr()) == (True, -1, None)
     assert _memory_state() == before
+
+
+@pytest.mark.parametrize("n", [777, sa.STATIC_CHECK_MAX])
+def test_a_call_takes_nothing_from_the_librarys_pool(n):
+    """The library's own pool keeps memory between calls, so an allocation from it would change none of the figures
+    above: its high-water mark shows the allocating check's use and none of this one's."""
+    text = W.natural_text(n, seed=15)
+    d_text = _device(text)
+    d_sa = _device(oracle.doubling_sa(text).astype(np.uint32))
+    library = ctypes.CDLL(str(harness()))
+    high = (ctypes.c_uint64 * 2)()
+    assert library.pool_use_of_checks(ctypes.c_void_p(d_text.data_ptr()), ctypes.c_int64(n),
+                                      ctypes.c_void_p(d_sa.data_ptr()), high) == 0
+    assert high[0] >= 4 * n and high[1] == 0
