@@ -238,7 +238,8 @@ int sadcs_gpu_check_bwt(const uint8_t* d_text, int64_t n, const uint8_t* d_bwt, 
  * n up to 2^32 - 256 (uint32 entries; the reference's int32 array views the same bytes): text (n
  * bytes, no padding needed) and sa (n entries) are copied to the device and checked there by
  * sadcs_gpu_check_suffix_array. *bad_index and *reason as there (CheckResult's index and reason).
- * Uses 9n bytes of temporary device memory. Returns SADCS_OK whenever the check ran. */
+ * Uses 9n bytes of temporary device memory, and from 16M entries on 8n more where they are to be had.
+ * Returns SADCS_OK whenever the check ran. */
 int sadcs_gpu_check_suffix_array_host(const uint8_t* text, int64_t n, const uint32_t* sa, int64_t* bad_index,
                                       const char** reason);
 
@@ -249,7 +250,8 @@ int sadcs_gpu_check_suffix_array_host(const uint8_t* text, int64_t n, const uint
 int sadcs_gpu_check_bwt_host(const uint8_t* text, int64_t n, const uint8_t* bwt, int64_t primary, int64_t* bad_index);
 
 /* No counterpart: the inverse BWT (unbwt) on the device: d_text (n bytes) from d_bwt and primary.
- * Returns SADCS_FAILED if d_bwt is not a valid BWT. */
+ * Returns SADCS_FAILED if d_bwt is not a valid BWT; the contents of d_text are unspecified then, nothing
+ * else is written. Uses about 7n bytes of temporary device memory. */
 int sadcs_gpu_inverse_bwt(const uint8_t* d_bwt, int64_t n, int64_t primary, uint8_t* d_text, void* stream);
 
 /* No counterpart (the reference computes no LCP array): the longest-common-prefix array of a suffix
@@ -257,8 +259,8 @@ int sadcs_gpu_inverse_bwt(const uint8_t* d_bwt, int64_t n, int64_t primary, uint
  * d_sa[r - 1] and d_sa[r], for d_sa (n uint32 entries) the suffix array of d_text (n bytes, no
  * padding needed), n up to 2^32 - 256. d_lcp gets n uint32 entries and may be d_sa itself (the
  * suffix array is then replaced by its LCP array). Uses about 4.13n bytes of temporary device memory,
- * and from 16M entries on 8n more where they are to be had; returns when the array is complete. A d_sa that is not the suffix array of d_text gives an
- * unspecified d_lcp, never a read outside the buffers. */
+ * and from 16M entries on 8n more where they are to be had; returns when the array is complete. A d_sa
+ * that is not the suffix array of d_text gives an unspecified d_lcp, never a read outside the buffers. */
 int sadcs_gpu_lcp(const uint8_t* d_text, int64_t n, const uint32_t* d_sa, uint32_t* d_lcp, void* stream);
 
 /* No counterpart: a test of the failure path of the radix passes' bounded wait (the decoupled

@@ -1,8 +1,8 @@
 """Builds libsadcs_gpu.so (sm_100a) in-tree with nvcc.
 
 ``python -m sadcs_b200.build`` or ``sadcs_b200.build.build_library()``. The library is a single
-translation unit (csrc/sadcs_gpu.cu includes the phase headers), so the __constant__ cover tables
-need no relocatable device code.
+translation unit (csrc/sadcs_gpu.cu includes the phase headers), so it needs no relocatable device
+code.
 """
 from __future__ import annotations
 

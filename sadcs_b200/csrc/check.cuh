@@ -97,7 +97,8 @@ __global__ void __launch_bounds__(kVerifyThreads) checkFirst(const uint8_t* __re
 // owned), and neighbours of the same first character (by starts; checkFirst says that they have it) in
 // order by the inverse of the suffix after it. Bound by its one random read per entry, isa[sa[i]] with
 // the entry after it (usually the same sector): read once and handed to the entry before by the warp,
-// the last lane's by memory. The characters read here too made it 4.5 ms at 128 MiB.
+// the last lane's by memory. 2.4 ms at 128 MiB; with the characters read here too, instead of by checkFirst (0.26 ms),
+// check and gather took 8.2 ms a call against 6.6.
 __global__ void __launch_bounds__(kVerifyThreads) checkVerify(const uint32_t* __restrict__ sa, uint32_t n,
                                                               const uint32_t* __restrict__ isa,
                                                               const uint32_t* __restrict__ starts,
@@ -154,8 +155,8 @@ namespace sadcs {
 // characters go to a buffer in chunks of 16 as they come (a chunk's piece and index beside it), because
 // a piece's place in the text is known only when all lengths are. Pointer jumping over the pieces
 // (n / kInverseStride of them) then gives the characters from each piece to the end, and a last pass
-// moves the chunks to their places. At 64 MiB of natural-language-like text the walk takes 1.9 of 2.7 ms
-// on the device: 36 G random 4-byte reads a second, against 62 ms for pointer jumping over every row
+// moves the chunks to their places. At 64 MiB of natural-language-like text the walk takes 2.0 of 2.8 ms
+// on the device: 34 G random 4-byte reads a second, against 62 ms for pointer jumping over every row
 // (27 rounds). A splitter in 64 or 256 rows costs 0.3-0.4 ms more than one in 128: more pieces to
 // order, or longer last pieces.
 constexpr uint32_t kInverseStride = 128;
@@ -266,7 +267,8 @@ __global__ void __launch_bounds__(kWalkThreads) inverseWalk(const uint32_t* __re
 
 // One round of pointer jumping for one piece: where the piece after it leads, the lengths added (mod 2^32).
 __host__ __device__ __forceinline__ uint64_t jumpOver(uint64_t mine, uint64_t next) {
-    return (next & 0xFFFFFFFF00000000ull) | static_cast<uint32_t>(static_cast<uint32_t>(mine) + static_cast<uint32_t>(next));
+    const uint32_t length = static_cast<uint32_t>(mine) + static_cast<uint32_t>(next);
+    return (next & 0xFFFFFFFF00000000ull) | length;
 }
 
 // One round of pointer jumping over the pieces and the end.

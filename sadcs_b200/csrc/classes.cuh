@@ -296,9 +296,9 @@ __global__ void __launch_bounds__(256) classHistogram(uint32_t total, TextSet te
     for (int i = threadIdx.x; i < kClasses * 256; i += blockDim.x) h[i] = 0;
     __syncthreads();
     const uint32_t b = texts.bits;
-    const uint64_t first = one ? static_cast<uint64_t>(blockIdx.x) * blockDim.x * 8 : static_cast<uint64_t>(blockIdx.x) * kHistChars;
+    const uint64_t first = static_cast<uint64_t>(blockIdx.x) * (one ? blockDim.x * 8 : kHistChars);
     const uint64_t stop = one ? total : min(static_cast<uint64_t>(total), first + kHistChars);
-    const uint64_t stride = one ? static_cast<uint64_t>(gridDim.x) * blockDim.x * 8 : static_cast<uint64_t>(blockDim.x) * 8;
+    const uint64_t stride = static_cast<uint64_t>(one ? gridDim.x : 1) * blockDim.x * 8;
     const uint32_t mine = texts.textOf(static_cast<uint32_t>(min(first, static_cast<uint64_t>(total))));
     for (uint64_t base = first + threadIdx.x * 8; base < stop; base += stride) {
         const uint64_t chunk = streamBits(texts.packed, base * b);
@@ -353,7 +353,8 @@ __global__ void __launch_bounds__(256) classHistogramPairs(uint32_t total, Class
 #pragma unroll
         for (int d = 1; d < kClasses; d++) {
             const uint64_t m = masks.mask[d] & inside;
-            const uint32_t all = __popcll(m), l = __popcll(m & low), g = __popcll(m & high), both = __popcll(m & low & high);
+            const uint32_t all = __popcll(m), l = __popcll(m & low), g = __popcll(m & high);
+            const uint32_t both = __popcll(m & low & high);
             count[d][3] += both;
             count[d][2] += g - both;
             count[d][1] += l - both;
@@ -441,9 +442,11 @@ inline cudaError_t sortClasses(uint32_t total, const TextSet& texts, const uint3
     SADCS_TRY(cudaMemsetAsync(radix.control, 0, 8, stream));
     if (J == 1 && texts.bits == 2) {
         const uint32_t blocks = std::min<uint32_t>(ceilDiv(total + 31ull, 32 * 256 * 4), 148 * 8);
-        SADCS_TRY(launch(classHistogramPairs, std::max(blocks, 1u), 256, 0, stream, total, classMasks(), texts.packed, hist));
+        SADCS_TRY(launch(classHistogramPairs, std::max(blocks, 1u), 256, 0, stream, total, classMasks(), texts.packed,
+                         hist));
     } else {
-        const uint32_t blocks = J == 1 ? std::min<uint32_t>(ceilDiv(total + 7ull, 256 * 8 * 8), 148 * 8) : ceilDiv(total, kHistChars);
+        const uint32_t blocks = J == 1 ? std::min<uint32_t>(ceilDiv(total + 7ull, 256 * 8 * 8), 148 * 8)
+                                       : ceilDiv(total, kHistChars);
         SADCS_TRY(launch(classHistogram, std::max(blocks, 1u), 256, 0, stream, total, texts, hist));
     }
     SADCS_TRY(launch(classDigitBase, kClasses * J, 256, 0, stream, hist, tables.rowBase));

@@ -228,7 +228,7 @@ inline size_t scratchWords(uint64_t n, bool pairs = false) {
     return pairs ? words + words % 2 + 2 * n + kMaxSlices : words;
 }
 
-// Arrays past the L2's size take their Phi by slices: at 128 MiB 2.0 ms (partition and scatter)
+// Arrays past the L2's size take their Phi by slices: at 128 MiB 1.7 ms (partition and scatter)
 // against 5.35 ms for the one-pass scatter, whose every write is a sector of DRAM read and written;
 // below it the one pass writes L2 (tuning).
 #ifndef SADCS_SLICED_SCATTER_MIN
@@ -250,9 +250,9 @@ inline cudaError_t lcpArray(const uint8_t* text, uint32_t n, const uint32_t* sa,
     const uint32_t longBlocks = std::min<uint32_t>(ceilDiv(words, kThreads / 32), 148u * 8);
     const bool aligned = (reinterpret_cast<uintptr_t>(text) & 7) == 0;
     if (pairs) {
-        const size_t words = scratchWords(n) + scratchWords(n) % 2;
-        uint64_t* pairWords = reinterpret_cast<uint64_t*>(scratch + words);
-        SADCS_TRY(scatterBySlices(PhiPairs{sa, n}, n, phiV, pairWords, scratch + words + 2 * static_cast<size_t>(n), stream));
+        uint32_t* pairWords = scratch + scratchWords(n) + scratchWords(n) % 2;  // two words a pair, then the fills
+        SADCS_TRY(scatterBySlices(PhiPairs{sa, n}, n, phiV, reinterpret_cast<uint64_t*>(pairWords),
+                                  pairWords + 2 * static_cast<size_t>(n), stream));
     } else {
         SADCS_TRY(launch(lcpPhi, blocks, kThreads, 0, stream, sa, n, phiV));
     }

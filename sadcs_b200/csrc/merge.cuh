@@ -365,12 +365,13 @@ inline cudaError_t copyDown(const OverlappedDownload& d, uint64_t from, uint64_t
 }
 
 // Merges the class lists of the texts into sa and/or bwt (either may be null). splitters and rows
-// are scratch sized by planMerge; counter is one device word (scratch); wide: the kernel for texts with few long repeats; rowZero and outBase are per
-// text (rowZero is filled here when a BWT is asked for); rowBase: the class tables' row bases.
-inline cudaError_t mergeClasses(uint32_t span, bool wide, const uint32_t* ranks, const TextSet& texts, const uint32_t* lists,
-                                const MergePlan& plan, const uint32_t* rowBase, const uint32_t* outBase,
-                                uint32_t* rowZero, uint32_t* splitters, MergeRow* rows, uint32_t* sa, uint8_t* bwt,
-                                uint32_t* counter, uint32_t* hostWord, cudaStream_t stream,
+// are scratch sized by planMerge; counter is one device word (scratch); positions are below span; wide: the
+// kernel for texts with few long repeats; rowZero and outBase are per text (rowZero is filled here when a BWT
+// is asked for); rowBase: the class tables' row bases.
+inline cudaError_t mergeClasses(uint32_t span, bool wide, const uint32_t* ranks, const TextSet& texts,
+                                const uint32_t* lists, const MergePlan& plan, const uint32_t* rowBase,
+                                const uint32_t* outBase, uint32_t* rowZero, uint32_t* splitters, MergeRow* rows,
+                                uint32_t* sa, uint8_t* bwt, uint32_t* counter, uint32_t* hostWord, cudaStream_t stream,
                                 cudaEvent_t finalStart = nullptr, cudaEvent_t finalStop = nullptr,
                                 uint32_t* const* saTexts = nullptr, uint8_t* const* bwtTexts = nullptr,
                                 const uint64_t* carried = nullptr, const OverlappedDownload* download = nullptr) {

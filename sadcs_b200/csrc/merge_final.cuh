@@ -1,5 +1,6 @@
 // merge_final.cuh - the merge levels (texts whose codes take more than one record word and that have few
-// long repeats go to merge_wide.cuh instead: useWideMerge): every tile of the 7 lists of a level merged in shared memory;
+// long repeats go to merge_wide.cuh instead: useWideMerge): every tile of the 7 lists of a level merged in
+// shared memory;
 // the last level writes the suffix array and the BWT, an upper level the rows of the level below.
 //
 // A tile's window set (at most kMergeCap records, merge.cuh) is held as arrays of fields, not as

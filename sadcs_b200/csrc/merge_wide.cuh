@@ -342,7 +342,8 @@ __global__ void __launch_bounds__(SADCS_WIDE_THREADS, SADCS_WIDE_TILES) mergeWid
             }
             const uint32_t x = p[first + j];
             const uint64_t bit = static_cast<uint64_t>(x) * bits;
-            const ulonglong2* src = reinterpret_cast<const ulonglong2*>(texts.packed) + min((bit + prefix.bits) >> 7, endUnit);
+            const uint64_t unit = min((bit + prefix.bits) >> 7, endUnit);
+            const ulonglong2* src = reinterpret_cast<const ulonglong2*>(texts.packed) + unit;
             w0[j] = __ldg(src);
             w1[j] = __ldg(src + 1);
             if constexpr (kFinal) c[j] = x ? charCode(texts, x - 1) : 0;

@@ -458,7 +458,8 @@ struct LoaderCarries<Loader, std::void_t<decltype(Loader::kCarry)>> {
 // natural-language-like text 16.9 -> 17.3; by the rule 2.69, 58.3, 0.42 and 16.5
 // (a share of 128 sends the protein-like text's digits to the match: 2.99). The class passes' few
 // digits match (2 GiB of genome-like text: 49.1 ms, 53.4 with votes).
-constexpr uint32_t kVoteShare = SADCS_VOTE_SHARE;  // votes where two random keys share a digit in fewer than 1 of kVoteShare cases
+// Votes where two random keys share a digit in fewer than 1 of kVoteShare cases.
+constexpr uint32_t kVoteShare = SADCS_VOTE_SHARE;
 __device__ __forceinline__ uint32_t digitPeers(uint32_t digit, bool valid) {
     uint32_t peers = __ballot_sync(0xffffffffu, valid);
 #pragma unroll
@@ -481,12 +482,10 @@ struct LoaderVotes<Loader, std::void_t<decltype(std::declval<const Loader&>().vo
 };
 
 template <class Key, class Loader, class Storer, class Segments = OneSegment>
-__global__ void __launch_bounds__(kSortThreads, SortTilesPerSm<Loader, Segments>::value) radixOnesweep(Loader ld, Storer st, Segments segs,
-                                                                 const uint32_t* __restrict__ digitBase,
-                                                                 uint32_t* __restrict__ status,
-                                                                 uint32_t* __restrict__ tileCounter,
-                                                                 uint32_t* __restrict__ error,
-                                                                 long long lookbackLimit) {
+__global__ void __launch_bounds__(kSortThreads, SortTilesPerSm<Loader, Segments>::value)
+    radixOnesweep(Loader ld, Storer st, Segments segs, const uint32_t* __restrict__ digitBase,
+                  uint32_t* __restrict__ status, uint32_t* __restrict__ tileCounter, uint32_t* __restrict__ error,
+                  long long lookbackLimit) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr bool kCarry = LoaderCarries<Loader>::value;
     constexpr bool kVotes = LoaderVotes<Loader>::value && std::is_same<Segments, OneSegment>::value;

@@ -106,8 +106,9 @@ inline cudaError_t rankFirstSort(const TextSet& texts, uint32_t count, int keyBi
     for (int p = 0; p < passes; p++) {
         const SortStorer<uint64_t> st{keysAlt, valsAlt, count};
         if (p == 0) {
-            SADCS_TRY((radixOnesweepPass<uint64_t>(FirstKeyLoader{FirstKeys{texts}, scratch.control + 8}, st, OneSegment{count}, count,
-                                                   ceilDiv(count, kSortTile), scratch.digitBase, scratch, stream)));
+            const FirstKeyLoader ld{FirstKeys{texts}, scratch.control + 8};
+            SADCS_TRY((radixOnesweepPass<uint64_t>(ld, st, OneSegment{count}, count, ceilDiv(count, kSortTile),
+                                                   scratch.digitBase, scratch, stream)));
         } else {
             const SortLoader<uint64_t> ld{keys, vals, 8 * p, scratch.control + 8 + p};
             SADCS_TRY((radixOnesweepPass<uint64_t>(ld, st, OneSegment{count}, count, ceilDiv(count, kSortTile),

@@ -724,7 +724,7 @@ int construct(sadcs_gpu_context* c, const Batch& b, Io& io, cudaStream_t stream,
 
     // The alphabet and the packed code stream.
     phase.next("sadcs ranking");
-    const uint64_t scanned = J == 1 ? b.end[0] : b.end[J - 1];
+    const uint64_t scanned = b.end[J - 1];
     if ((error = prepareAlphabet(text, scanned, b.span, reinterpret_cast<uint32_t*>(slab + L.alphabet),
                                  c->hostWords + c->hostWordCount - 256, reinterpret_cast<uint64_t*>(slab + L.packed),
                                  texts, stream)) != cudaSuccess) {
@@ -775,7 +775,7 @@ int construct(sadcs_gpu_context* c, const Batch& b, Io& io, cudaStream_t stream,
     uint64_t* carried = L.carried && carriesWords(texts) && b.outputs >= carryMinBytes()
                             ? reinterpret_cast<uint64_t*>(slab + L.carried)
                             : nullptr;
-    if ((error = sortClasses(J == 1 ? b.end[0] : b.end[J - 1], texts, ranks, static_cast<uint32_t>(b.slots), b.classes,
+    if ((error = sortClasses(b.end[J - 1], texts, ranks, static_cast<uint32_t>(b.slots), b.classes,
                              classTables, lists, classScratch, chains, carried, stream)) != cudaSuccess) {
         return failed("class sorts", error);
     }
@@ -797,7 +797,8 @@ int construct(sadcs_gpu_context* c, const Batch& b, Io& io, cudaStream_t stream,
     uint32_t* sa = saPieces ? nullptr
                             : (io.outSa ? io.outSa : (io.wantSa ? reinterpret_cast<uint32_t*>(slab + L.sa) : nullptr));
     uint8_t* bwt = bwtPieces ? nullptr : (io.outBwt ? io.outBwt : (io.wantBwt ? slab + L.bwt : nullptr));
-    // The merge's kernel and tile shape follow the code width and the ties, known now (the memory plan bounds every shape).
+    // The merge's kernel and tile shape follow the code width and the ties, known now (the memory plan bounds
+    // every shape).
     const bool wide = useWideMerge(texts.bits, rankStats.ties, b.live);
     if (traceEnabled()) {
         fprintf(stderr, "sadcs: merge %s, %llu of %llu samples tied\n", wide ? "wide" : "tree",
@@ -816,8 +817,8 @@ int construct(sadcs_gpu_context* c, const Batch& b, Io& io, cudaStream_t stream,
         download.hostRows = c->hostWords + 64;  // the tables' staging words, free since their upload
         download.outputs = b.outputs;
     }
-    if ((error = mergeClasses(J == 1 ? b.end[0] : b.end[J - 1], wide, ranks, texts, lists, mergePlan, classTables.rowBase, dOutBase, dRowZero,
-                              reinterpret_cast<uint32_t*>(slab + L.splitters),
+    if ((error = mergeClasses(b.end[J - 1], wide, ranks, texts, lists, mergePlan, classTables.rowBase, dOutBase,
+                              dRowZero, reinterpret_cast<uint32_t*>(slab + L.splitters),
                               reinterpret_cast<MergeRow*>(slab + L.rows), sa, bwt,
                               reinterpret_cast<uint32_t*>(slab + L.mergeCounter), c->hostWords, stream,
                               c->events[4], c->events[5], saPieces, bwtPieces, carried,
@@ -1179,7 +1180,9 @@ int sadcs_gpu_bwt_from_sa(const uint8_t* d_text, int64_t n, const uint32_t* d_sa
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint32_t* word = nullptr;
     cudaError_t error;
-    if ((error = workspace(&word, sizeof(uint32_t), st)) != cudaSuccess) return failed("allocating the gather's word", error);
+    if ((error = workspace(&word, sizeof(uint32_t), st)) != cudaSuccess) {
+        return failed("allocating the gather's word", error);
+    }
     uint32_t row0 = 0;
     error = bwtFromSa(d_text, static_cast<uint32_t>(n), d_sa, d_bwt, word, st, &row0);
     cudaFreeAsync(word, st);
@@ -1207,7 +1210,9 @@ int sadcs_gpu_check_suffix_array(const uint8_t* d_text, int64_t n, const uint32_
     uint64_t* pairs = nullptr;
     unsigned long long host[3] = {kNoFailure, kNoFailure, kNoFailure};
     cudaError_t error;
-    if ((error = workspace(&isa, 4 * static_cast<size_t>(n), st)) != cudaSuccess) return failed("allocating check buffers", error);
+    if ((error = workspace(&isa, 4 * static_cast<size_t>(n), st)) != cudaSuccess) {
+        return failed("allocating check buffers", error);
+    }
     if ((error = workspace(&words, 4 * sizeof(unsigned long long) + 256 * sizeof(uint32_t), st)) != cudaSuccess) {
         cudaFreeAsync(isa, st);
         return failed("allocating check buffers", error);
@@ -1232,9 +1237,16 @@ int sadcs_gpu_check_suffix_array(const uint8_t* d_text, int64_t n, const uint32_
     const uint32_t stridedBlocks = std::min<uint32_t>(ceilDiv(count, 256 * 16), 148 * 8);
     if (error == cudaSuccess) error = launch(byteHistogram, stridedBlocks, 256, 0, st, d_text, count, starts);
     if (error == cudaSuccess) error = launch(inverseChunkBases, 1, 256, 0, st, starts, 1u);
-    if (error == cudaSuccess) error = launch(checkFirst, stridedBlocks, kVerifyThreads, 0, st, d_text, count, isa, starts, failedWord);
-    if (error == cudaSuccess) error = launch(checkVerify, ceilDiv(count, kVerifyThreads), kVerifyThreads, 0, st, d_sa, count, isa, starts, failedWord);
-    if (error == cudaSuccess) error = cudaMemcpyAsync(&hostFailed, failedWord, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+    if (error == cudaSuccess) {
+        error = launch(checkFirst, stridedBlocks, kVerifyThreads, 0, st, d_text, count, isa, starts, failedWord);
+    }
+    if (error == cudaSuccess) {
+        error = launch(checkVerify, ceilDiv(count, kVerifyThreads), kVerifyThreads, 0, st, d_sa, count, isa, starts,
+                       failedWord);
+    }
+    if (error == cudaSuccess) {
+        error = cudaMemcpyAsync(&hostFailed, failedWord, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+    }
     if (error == cudaSuccess) error = cudaStreamSynchronize(st);
     const char* why = nullptr;
     int64_t index = -1;

@@ -28,7 +28,9 @@ namespace sadcs {
 #endif
 
 #ifndef SADCS_SEGSORT_SMALL
-#define SADCS_SEGSORT_SMALL 1024  // largest segment sorted in shared memory (tuning; 1024 with 4 blocks per SM: 1.4 ms less ranking at 256 MiB than 2048 with 2)
+// Largest segment sorted in shared memory (tuning; 1024 with 4 blocks per SM: 1.4 ms less ranking at 256 MiB than
+// 2048 with 2).
+#define SADCS_SEGSORT_SMALL 1024
 #endif
 
 constexpr uint32_t kSegSmall = SADCS_SEGSORT_SMALL;  // largest segment sorted in one block
@@ -232,8 +234,8 @@ constexpr uint32_t kDirectSample = 64;
 __host__ __device__ __forceinline__ bool directWorthwhile(uint32_t compared, uint32_t decided) {
     return static_cast<uint64_t>(decided) * kDirectShare >= compared;
 }
-__host__ __device__ __noinline__ int directOrder(const uint64_t* __restrict__ packed, uint32_t b, uint32_t end, uint32_t i,
-                                                 uint32_t j, uint32_t from) {
+__host__ __device__ __noinline__ int directOrder(const uint64_t* __restrict__ packed, uint32_t b, uint32_t end,
+                                                 uint32_t i, uint32_t j, uint32_t from) {
     const uint32_t perWord = 64 / b, shorter = end - (i > j ? i : j);  // characters of the shorter suffix
     uint64_t at = from;
     for (int w = 0; w < SADCS_DIRECT_WORDS; w++, at += perWord) {
@@ -250,7 +252,8 @@ __host__ __device__ __noinline__ int directOrder(const uint64_t* __restrict__ pa
 // exchanges of neighbours. equal, bit i: elements i and i + 1 have the same key. Returns it without the
 // bits of neighbours that are now known to differ.
 template <class Order>
-__host__ __device__ __forceinline__ uint32_t orderEqual(uint32_t (&val)[kSegTiny], uint32_t size, uint32_t equal, Order order) {
+__host__ __device__ __forceinline__ uint32_t orderEqual(uint32_t (&val)[kSegTiny], uint32_t size, uint32_t equal,
+                                                        Order order) {
     uint32_t same = equal;
     for (uint32_t round = 1; round < size; round++) {  // until a round exchanges nothing
         bool exchanged = false;
@@ -288,7 +291,8 @@ __host__ __device__ __forceinline__ uint32_t orderEqual(uint32_t (&val)[kSegTiny
 template <bool kDirect>
 __global__ void __launch_bounds__(256) segSortTiny(const uint32_t* __restrict__ heads, uint32_t segments, TextSet texts,
                                                    uint32_t depth, uint64_t* __restrict__ keys,
-                                                   uint32_t* __restrict__ vals, uint32_t* __restrict__ direct, bool sampled) {
+                                                   uint32_t* __restrict__ vals, uint32_t* __restrict__ direct,
+                                                    bool sampled) {
     uint32_t block = blockIdx.x;
     bool compare = false;
     if constexpr (kDirect) {
@@ -384,9 +388,9 @@ __global__ void segCopyBack(ListSegments segs, const uint64_t* __restrict__ kFro
 // elements are spread evenly over the warps. The ranking of a 48 MiB text of versions of one document
 // took 16.7 ms with every pass made over the block's first warps, 13.6 now (of it 1.5 by the direct
 // rank writes of small arrays), of 256 MiB of natural-language-like text 17.8 and 16.9.
-__global__ void __launch_bounds__(kSegThreads, SADCS_SEGSORT_BLOCKS) segSortSmall(const uint32_t* __restrict__ heads, uint32_t segments,
-                                                            const uint64_t* keyIn, const uint32_t* valIn,
-                                                            uint64_t* keyOut, uint32_t* valOut, int keyBits) {
+__global__ void __launch_bounds__(kSegThreads, SADCS_SEGSORT_BLOCKS)
+    segSortSmall(const uint32_t* __restrict__ heads, uint32_t segments, const uint64_t* keyIn, const uint32_t* valIn,
+                 uint64_t* keyOut, uint32_t* valOut, int keyBits) {
     extern __shared__ __align__(16) unsigned char smem[];
     uint64_t* sKey = reinterpret_cast<uint64_t*>(smem);                 // kSegCap
     uint32_t* sVal = reinterpret_cast<uint32_t*>(sKey + kSegCap);       // kSegCap
